@@ -88,12 +88,16 @@ enum : uint32_t {
 IBS_HD bool is_mz(uint32_t fmt) { return fmt == FMT_MZ8 || fmt == FMT_MZ6; }
 constexpr uint32_t B8_EMPTY = 0xffffffffu;
 constexpr uint32_t B8_OVERFLOW = 0xfffffffeu;
-// Minimizer lines of B8x32 sectors (MZ8) keep a full sector's extra keys in
-// its partner sector of the same line (index ^ 1) while that has free slots:
-// slot 7 = B8_OVERFLOW says the extras are all there, B8_OVERFLOW_STASH that
-// some went on to the stash. (A slot value identifies its k-mer inside the
-// whole line, so the two sectors' keys never collide.)
-constexpr uint32_t B8_OVERFLOW_STASH = 0xfffffffdu;
+// Minimizer lines (MZ8, MZ6) keep a full sector's extra keys in the line's
+// other sectors while those have free slots: how far they went is the
+// sector's reach (0: nowhere, 1: its partner, index ^ 1, only; 2: any sector
+// of the line; 3: the stash too). MZ8 says so in slot 7, with the sentinels
+// below EMPTY (0xffffffff - reach), and MZ6 in the flag byte. A slot value
+// identifies its k-mer inside the whole line, so the sectors' keys never
+// collide.
+constexpr uint32_t B8_REACH_3 = 0xfffffffcu;
+IBS_HD uint32_t mz8_reach(uint32_t word7) { return word7 >= B8_REACH_3 ? 0xffffffffu - word7 : 0u; }
+IBS_HD uint32_t mz6_reach(uint32_t word7) { return (word7 >> 24) & 3u; }
 constexpr uint64_t STASH_EMPTY = ~0ull;
 
 struct TableGeom {

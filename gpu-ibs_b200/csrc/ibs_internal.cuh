@@ -132,47 +132,79 @@ __device__ __forceinline__ uint32_t bucket_match(const uint4 &v0, const uint4 &v
     }
 }
 
-// An MZ8 sector compare: 1 on a hit, 0 on a sure miss, 2 when the sector's
-// extra keys are in its partner sector, 3 when also in the stash.
-__device__ __forceinline__ uint32_t mz8_match(const uint4 &v0, const uint4 &v1, uint32_t slot)
+// A 32-byte sector in one load (two 16-byte loads ask the L1 twice; with many
+// probes in flight random sectors came at 25 to 34 G/s so, at 36.4 G/s with
+// one load each, whatever is in flight).
+__device__ __forceinline__ void load_sector(const uint4 *p, uint4 &a, uint4 &b)
 {
-    const bool hit = (v0.x == slot) | (v0.y == slot) | (v0.z == slot) | (v0.w == slot) | (v1.x == slot) |
-                     (v1.y == slot) | (v1.z == slot) | (v1.w == slot);
-    return hit ? 1u : (v1.w == B8_OVERFLOW ? 2u : (v1.w == B8_OVERFLOW_STASH ? 3u : 0u));
+    asm volatile("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
+                 : "l"(p));
 }
 
-// The rest of an MZ8 probe whose sector r reported m >= 2: the partner
-// sector r ^ 1 of the same line, then (m == 3) the stash.
-__device__ __forceinline__ bool mz8_overflow_lookup(const TableView &t, uint64_t r, uint32_t slot, uint32_t m,
-                                                    uint64_t code)
+// Whether a minimizer line's sector holds a slot value. B6x40: each slot's
+// 32-bit half by one comparison and its byte by one masked difference; the
+// slots past the count hold zeros, which only a slot value of zero can match.
+template <uint32_t SEC>
+__device__ __forceinline__ bool mz_sector_holds(const uint4 &v0, const uint4 &v1, uint32_t slot, uint32_t high)
 {
-    const uint4 w0 = __ldg(t.buckets + 2 * (r ^ 1)), w1 = __ldg(t.buckets + 2 * (r ^ 1) + 1);
-    if ((w0.x == slot) | (w0.y == slot) | (w0.z == slot) | (w0.w == slot) | (w1.x == slot) | (w1.y == slot) |
-        (w1.z == slot) | (w1.w == slot))
-        return true;
-    return m == 3u && stash_lookup(t, code);
+    if (SEC == FMT_B8X32)
+        return (v0.x == slot) | (v0.y == slot) | (v0.z == slot) | (v0.w == slot) | (v1.x == slot) | (v1.y == slot) |
+               (v1.z == slot) | (v1.w == slot);
+    const uint32_t qhi = __funnelshift_r(slot, high, 8), qlo = slot & 0xffu;
+    const uint32_t rep = qlo * 0x01010101u, d0 = v1.z ^ rep, d1 = v1.w ^ rep;
+    bool hit = v0.x == qhi && !(d0 & 0x000000ffu);
+    hit |= v0.y == qhi && !(d0 & 0x0000ff00u);
+    hit |= v0.z == qhi && !(d0 & 0x00ff0000u);
+    hit |= v0.w == qhi && !(d0 & 0xff000000u);
+    hit |= v1.x == qhi && !(d1 & 0x000000ffu);
+    hit |= v1.y == qhi && !(d1 & 0x0000ff00u);
+    if ((qhi | qlo) == 0)
+        hit = bucket_match<FMT_B6X40>(v0, v1, 0) == 1u;
+    return hit;
+}
+
+template <uint32_t SEC> __device__ __forceinline__ uint32_t mz_reach(const uint4 &v1)
+{
+    return SEC == FMT_B8X32 ? mz8_reach(v1.w) : mz6_reach(v1.w);
+}
+
+// The rest of a minimizer-line probe that its sector r (of reach > 0) does
+// not hold: sectors r ^ 1, then r ^ 2 and r ^ 3 of the same line (the stash
+// is next). 16-byte loads: ptxas 12.9 crashes on 32-byte ones in the
+// functions kept out of line that this goes into.
+template <uint32_t SEC>
+__device__ __forceinline__ bool mz_line_holds(const TableView &t, uint64_t r, uint32_t reach, uint32_t slot,
+                                              uint32_t high)
+{
+    auto holds = [&](uint64_t x) {
+        return mz_sector_holds<SEC>(__ldg(t.buckets + 2 * x), __ldg(t.buckets + 2 * x + 1), slot, high);
+    };
+    return holds(r ^ 1) || (reach > 1u && (holds(r ^ 2) || holds(r ^ 3)));
 }
 
 template <uint32_t FMT>
 __device__ __forceinline__ bool table_lookup(const TableView &t, uint64_t code)
 {
-    if (FMT == FMT_MZ8) {
+    if constexpr (FMT == FMT_MZ8 || FMT == FMT_MZ6) {
+        constexpr uint32_t SEC = FMT == FMT_MZ8 ? FMT_B8X32 : FMT_B6X40;
         uint64_t r, slot;
-        mz::locate(code, t.g, r, slot);
-        const uint4 v0 = __ldg(t.buckets + 2 * r), v1 = __ldg(t.buckets + 2 * r + 1);
-        const uint32_t m = mz8_match(v0, v1, (uint32_t)slot);
-        return m == 1u || (m >= 2u && mz8_overflow_lookup(t, r, (uint32_t)slot, m, code));
-    }
-    if (FMT == FMT_MZ6) {
-        uint64_t r, slot;
-        mz::locate(code, t.g, r, slot);
-        const uint4 v0 = __ldg(t.buckets + 2 * r), v1 = __ldg(t.buckets + 2 * r + 1);
-        const uint32_t m = bucket_match<FMT_B6X40>(v0, v1, slot);
-        return m == 1u || (m == 2u && stash_lookup(t, code));
+        if (!mz::locate(code, t.g, r, slot))
+            return stash_lookup(t, code);
+        const uint32_t lo = (uint32_t)slot, hi = (uint32_t)(slot >> 32);
+        uint4 v0, v1;
+        load_sector(t.buckets + 2 * r, v0, v1);
+        if (mz_sector_holds<SEC>(v0, v1, lo, hi))
+            return true;
+        const uint32_t reach = mz_reach<SEC>(v1);
+        if (!reach)
+            return false;
+        return mz_line_holds<SEC>(t, r, reach, lo, hi) || (reach == 3u && stash_lookup(t, code));
     }
     const uint64_t h = perm_hash(code, t.g.bits);
     const uint64_t r = bucket_of(h, t.g);
-    const uint4 v0 = __ldg(t.buckets + 2 * r), v1 = __ldg(t.buckets + 2 * r + 1);
+    uint4 v0, v1;
+    load_sector(t.buckets + 2 * r, v0, v1);
     const uint32_t m = bucket_match<FMT>(v0, v1, fp_of(h, t.g));
     return m == 1u || (m == 2u && stash_lookup(t, code));
 }

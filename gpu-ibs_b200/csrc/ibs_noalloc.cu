@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(256) k_na_spans(TableView t, const uint64_t *_
         const uint64_t base = cd[c].base + i * ((uint64_t)W - k);
         const uint32_t p0 = (uint32_t)sc * kSpanLen;
         const uint32_t p1 = (uint32_t)(p0 + kSpanLen < nPos ? p0 + kSpanLen : nPos);
-        dev::LaneFold fold;
+        dev::LaneFold<> fold;
         for (uint32_t p = p0; p < p1; p += 32 * NB) {
             uint4 v0[NB], v1[NB];
             uint64_t code[NB], fp[NB];

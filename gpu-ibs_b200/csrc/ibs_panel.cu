@@ -81,8 +81,8 @@ __device__ __forceinline__ bool claim_slot(uint32_t *w, uint32_t fp, uint32_t bi
 // ---- build: phase A finds keys already present and ORs in the sample bit;
 // phase B inserts the rest. Within one sample the keys are unique, so no
 // lookup races with an insert of the same key. A key is looked for where
-// phase B would have put it: its home sector, then (PM, flagged) the home's
-// partner sector, then (flagged) the stash.
+// phase B would have put it: its home sector, then (PM, flagged) the line's
+// others, then (flagged) the stash; a key with two places, at each.
 __global__ void k_find(View t, uint32_t *words, unsigned long long *stashWords, const uint64_t *codes,
                        uint64_t n, uint32_t bit, uint64_t *pending, unsigned long long *nPending)
 {
@@ -92,35 +92,44 @@ __global__ void k_find(View t, uint32_t *words, unsigned long long *stashWords, 
     const bool pm = t.g.format == FMT_PANEL_MZ;
     for (uint64_t it = 0; it < iters; ++it) {
         const uint64_t i = it * stride + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-        bool miss = false;
-        uint64_t code = 0;
+        uint64_t code = 0, r[2];
+        uint32_t fp[2], places = 0, turns = 0;
         if (i < n) {
             code = codes[i];
-            uint64_t r;
-            uint32_t fp;
-            joint_place(t, code, r, fp);
-            uint32_t *w = words + 8 * r;
-            const uint32_t flags = w[7];
-            int slot = find_slot(w, fp);
-            uint32_t *where = w;
-            if (slot < 0 && pm && (flags & kPartnerFlag)) {
-                where = words + 8 * (r ^ 1);
-                slot = find_slot(where, fp);
-            }
-            if (slot >= 0)
-                atomicOr(where + 5 + slot / 2, (1u << bit) << (16 * (slot & 1)));
-            else
-                miss = !((flags & kStashFlag) && stash_or(t, stashWords, code, bit));
+            places = joint_places(t, code, r, fp);
+            turns = places ? places : 1;
         }
-        const uint32_t ballot = __ballot_sync(0xffffffffu, miss);
-        if (!ballot)
-            continue;
-        unsigned long long base = 0;
-        if (lane == 0)
-            base = atomicAdd(nPending, (unsigned long long)__popc(ballot));
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (miss)
-            pending[base + __popc(ballot & ((1u << lane) - 1u))] = code;
+        for (uint32_t a = 0; __any_sync(0xffffffffu, a < turns); ++a) {
+            bool miss = false;
+            if (a < turns && !places) {
+                miss = !stash_or(t, stashWords, code, bit);
+            } else if (a < turns) {
+                const uint64_t ra = a ? r[1] : r[0];
+                const uint32_t fa = a ? fp[1] : fp[0];
+                uint32_t *w = words + 8 * ra;
+                const uint32_t flags = w[7];
+                int slot = find_slot(w, fa);
+                uint32_t *where = w;
+                for (uint32_t d = 1; d < 4 && slot < 0 && pm && (flags & (d == 1 ? kPartnerFlag : kLineFlag)); ++d) {
+                    where = words + 8 * (ra ^ d);
+                    slot = find_slot(where, fa);
+                }
+                if (slot >= 0)
+                    atomicOr(where + 5 + slot / 2, (1u << bit) << (16 * (slot & 1)));
+                else
+                    miss = !((flags & kStashFlag) && stash_or(t, stashWords, code, bit));
+            }
+            const uint32_t ballot = __ballot_sync(0xffffffffu, miss);
+            if (!ballot)
+                continue;
+            unsigned long long base = 0;
+            if (lane == 0)
+                base = atomicAdd(nPending, (unsigned long long)__popc(ballot));
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if (miss)
+                pending[base + __popc(ballot & ((1u << lane) - 1u))] =
+                    code | (!places ? mz::kNoPlace : a ? mz::kSecondPlace : 0ull);
+        }
     }
 }
 
@@ -130,19 +139,30 @@ __global__ void k_insert(View t, uint32_t *words, unsigned long long *stashWords
     const bool pm = t.g.format == FMT_PANEL_MZ;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
          i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t code = codes[i];
-        uint64_t r;
-        uint32_t fp;
-        joint_place(t, code, r, fp);
-        uint32_t *w = words + 8 * r;
-        if (claim_slot(w, fp, bit))
-            continue;
-        if (pm) { // the partner sector of the same line, flagged on the home sector
-            atomicOr(w + 7, kPartnerFlag);
-            if (claim_slot(words + 8 * (r ^ 1), fp, bit))
+        const uint64_t entered = codes[i];
+        const uint64_t code = pm ? entered & ~(mz::kSecondPlace | mz::kNoPlace) : entered;
+        if (!pm || !(entered & mz::kNoPlace)) {
+            uint64_t rr[2];
+            uint32_t ff[2];
+            joint_places(t, code, rr, ff);
+            const bool second = pm && (entered & mz::kSecondPlace);
+            const uint64_t r = second ? rr[1] : rr[0];
+            const uint32_t fp = second ? ff[1] : ff[0];
+            uint32_t *w = words + 8 * r;
+            if (claim_slot(w, fp, bit))
                 continue;
+            if (pm) { // the line's other sectors, flagged on the home sector
+                atomicOr(w + 7, kPartnerFlag);
+                bool claimed = claim_slot(words + 8 * (r ^ 1), fp, bit);
+                if (!claimed) {
+                    atomicOr(w + 7, kLineFlag);
+                    claimed = claim_slot(words + 8 * (r ^ 2), fp, bit) || claim_slot(words + 8 * (r ^ 3), fp, bit);
+                }
+                if (claimed)
+                    continue;
+            }
+            atomicOr(w + 7, kStashFlag);
         }
-        atomicOr(w + 7, kStashFlag);
         uint64_t b = stash_home(code, t.stashBuckets);
         bool placed = false;
         // at most kStashProbe buckets from home: a crowded stash fails the
@@ -162,7 +182,7 @@ __global__ void k_insert(View t, uint32_t *words, unsigned long long *stashWords
             b = (b + 1) & (t.stashBuckets - 1);
         }
         if (!placed) // the stash is full: the host grows it and inserts these again
-            failed[atomicAdd(nFailed, 1ull)] = code;
+            failed[atomicAdd(nFailed, 1ull)] = entered;
     }
 }
 
@@ -202,7 +222,21 @@ __global__ void k_stash_move(const ulonglong2 *old, uint64_t oldEntries, unsigne
 // one range.
 enum : int { kScan = 0, kMaskPass = 1, kStats = 2 };
 
-template <int NB, int MODE, bool PM>
+__device__ __forceinline__ uint32_t window_of(const uint32_t *__restrict__ span0, uint32_t nWin, uint64_t s)
+{
+    uint32_t lo = 0, hi = nWin - 1;
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi + 1) >> 1;
+        if (__ldg(span0 + mid) <= s)
+            lo = mid;
+        else
+            hi = mid - 1;
+    }
+    return lo;
+}
+
+// The hash-sector tables (P5x48), and the statistics pass of either layout.
+template <int NB, int MODE>
 __global__ void __launch_bounds__(256) k_panel_spans(View t, const uint64_t *__restrict__ seq,
                                                      const uint64_t *__restrict__ mask,
                                                      const WinDesc *__restrict__ win,
@@ -213,14 +247,10 @@ __global__ void __launch_bounds__(256) k_panel_spans(View t, const uint64_t *__r
                                                      SegStats *__restrict__ out, uint16_t *__restrict__ masks,
                                                      uint64_t bLo, uint64_t bHi, bool firstPass)
 {
-    // PM tables locate a k-mer through its minimizer (one block of m-mers
-    // read ahead); the statistics pass only needs each position's validity
-    constexpr bool kMz = PM && MODE != kStats;
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t k = t.g.k;
     const uint64_t kmask = key_mask(2 * k);
     const uint64_t kbits = (1ull << k) - 1;
-    const uint32_t w = kMz ? mz::w_of(k) : 1, m = kMz ? mz::m_of(k) : 0;
     for (;;) {
         unsigned long long s = 0;
         if (lane == 0)
@@ -228,71 +258,37 @@ __global__ void __launch_bounds__(256) k_panel_spans(View t, const uint64_t *__r
         s = __shfl_sync(dev::FULL_MASK, s, 0);
         if (s >= nSpans)
             break;
-        uint32_t lo = 0, hi = nWin - 1;
-        while (lo < hi) {
-            const uint32_t mid = (lo + hi + 1) >> 1;
-            if (__ldg(span0 + mid) <= s)
-                lo = mid;
-            else
-                hi = mid - 1;
-        }
+        const uint32_t lo = window_of(span0, nWin, s);
         const uint64_t base = win[lo].base;
         const uint32_t nPos = win[lo].nPos;
         const uint32_t p0 = (uint32_t)(s - __ldg(span0 + lo)) * spanLen;
         const uint32_t p1 = min(p0 + spanLen, nPos);
         uint16_t *spanMasks = masks + s * spanLen - p0; // position q of the span at spanMasks[q]
         SegStats acc = seg_empty(); // lane j < nSamples: sample j
-        // PM: the last m-mer start the window's k-mers use; lanes past the
-        // span read up to it (inside the window's bases) and are masked out
-        const uint32_t lastM = nPos - 1 + (w - 1);
-        dev::MzPos next;
-        if constexpr (kMz)
-            next = dev::mz_pos(seq, mask, base + min(p0 + lane, lastM), k, m);
         for (uint32_t p = p0; p < p1; p += 32 * NB) {
             uint4 v0[NB], v1[NB];
             uint64_t code[NB], rr[NB];
             uint32_t fp[NB];
             bool valid[NB], mine[NB];
-            if constexpr (kMz) {
-                dev::MzPos ps[NB + 1];
-                ps[0] = next;
 #pragma unroll
-                for (int b = 1; b <= NB; ++b)
-                    ps[b] = dev::mz_pos(seq, mask, base + min(p + 32 * b + lane, lastM), k, m);
-                next = ps[NB];
-#pragma unroll
-                for (int b = 0; b < NB; ++b) {
-                    const uint32_t q = p + 32 * b + lane;
-                    valid[b] = q < p1 && ps[b].acgt;
-                    uint64_t slot;
-                    dev::mz_locate_lane<true>(ps[b], ps[b + 1], lane, k, w, t.g.nBuckets, t.g.fpBits, rr[b], slot);
-                    fp[b] = (uint32_t)slot;
-                    code[b] = ps[b].code;
-                }
-            } else {
-#pragma unroll
-                for (int b = 0; b < NB; ++b) {
-                    const uint32_t q = p + 32 * b + lane;
-                    const bool inSpan = q < p1;
-                    const uint64_t G = base + (inSpan ? q : p0);
-                    bool acgt;
-                    code[b] = dev::canonical_at(seq, mask, G, k, kmask, kbits, acgt);
-                    valid[b] = inSpan && acgt;
-                    const uint64_t h = perm_hash(code[b], t.g.bits);
-                    rr[b] = bucket_of(h, t.g);
-                    fp[b] = (uint32_t)fp_of(h, t.g);
-                }
+            for (int b = 0; b < NB; ++b) {
+                const uint32_t q = p + 32 * b + lane;
+                const bool inSpan = q < p1;
+                const uint64_t G = base + (inSpan ? q : p0);
+                bool acgt;
+                code[b] = dev::canonical_at(seq, mask, G, k, kmask, kbits, acgt);
+                valid[b] = inSpan && acgt;
+                const uint64_t h = perm_hash(code[b], t.g.bits);
+                rr[b] = bucket_of(h, t.g);
+                fp[b] = (uint32_t)fp_of(h, t.g);
             }
 #pragma unroll
             for (int b = 0; b < NB; ++b) {
                 mine[b] = valid[b] && (MODE != kMaskPass || (rr[b] >= bLo && rr[b] < bHi));
-                if (MODE != kStats && mine[b]) {
-                    v0[b] = __ldg(t.buckets + 2 * rr[b]);
-                    v1[b] = __ldg(t.buckets + 2 * rr[b] + 1);
-                } else {
-                    v0[b] = make_uint4(0, 0, 0, 0);
-                    v1[b] = make_uint4(0, 0, 0, 0);
-                }
+                v0[b] = make_uint4(0, 0, 0, 0);
+                v1[b] = make_uint4(0, 0, 0, 0);
+                if (MODE != kStats && mine[b])
+                    load_sector(t.buckets + 2 * rr[b], v0[b], v1[b]);
             }
 #pragma unroll
             for (int b = 0; b < NB; ++b) {
@@ -302,13 +298,9 @@ __global__ void __launch_bounds__(256) k_panel_spans(View t, const uint64_t *__r
                     if (valid[b])
                         m = spanMasks[q];
                 } else if (mine[b]) {
-                    if constexpr (kMz) {
-                        m = pm_mask(t, v0[b], v1[b], rr[b], fp[b], code[b]);
-                    } else {
-                        m = bucket_mask(v0[b], v1[b], fp[b]);
-                        if (m & 0x80000000u)
-                            m = stash_mask(t, code[b]);
-                    }
+                    m = bucket_mask(v0[b], v1[b], fp[b]);
+                    if (m & 0x80000000u)
+                        m = stash_mask(t, code[b]);
                 }
                 if (MODE == kMaskPass) {
                     if (q < p1 && (firstPass || m))
@@ -328,6 +320,59 @@ __global__ void __launch_bounds__(256) k_panel_spans(View t, const uint64_t *__r
         }
         if (MODE != kMaskPass && lane < nSamples)
             out[(uint64_t)lane * nSpans + s] = acc;
+    }
+}
+
+// The minimizer-line tables (PM), k fixed at compile time: located 128
+// positions at a time as the single-sample scan (mz_scan.cuh), one sector
+// load a position, then kScan's statistics or kMaskPass's masks.
+template <uint32_t K, int MODE>
+__global__ void __launch_bounds__(256, 3) k_panel_spans_mz(const __grid_constant__ View t, const uint64_t *__restrict__ seq,
+                                                           const uint64_t *__restrict__ mask,
+                                                           const WinDesc *__restrict__ win,
+                                                           const uint32_t *__restrict__ span0, uint32_t nWin,
+                                                           uint64_t nSpans, uint32_t spanLen, uint32_t nSamples,
+                                                           unsigned long long *__restrict__ work,
+                                                           SegStats *__restrict__ out, uint16_t *__restrict__ masks,
+                                                           uint64_t bLo, uint64_t bHi, bool firstPass)
+{
+    __shared__ dev::MzShared<FMT_B8X32> shared[8];
+    dev::MzShared<FMT_B8X32> *sh = &shared[threadIdx.x >> 5];
+    const uint32_t lane = dev::lane_id();
+    for (;;) {
+        unsigned long long s = 0;
+        if (lane == 0)
+            s = atomicAdd(work, 1ull);
+        s = __shfl_sync(dev::FULL_MASK, s, 0);
+        if (s >= nSpans)
+            break;
+        const uint32_t w = window_of(span0, nWin, s);
+        const uint64_t base = win[w].base;
+        const uint32_t nPos = win[w].nPos;
+        const uint32_t p0 = (uint32_t)(s - __ldg(span0 + w)) * spanLen;
+        const uint32_t n = min(spanLen, nPos - p0);
+        dev::MzWarp<K, FMT_B8X32> warp(sh, t.g, seq, mask, base + p0, n, base + nPos - 1 + (K - 1), lane);
+        JointFold fold(lane);
+        warp.start();
+        for (int b = warp.blocks() - 1; b >= 0; --b) {
+            warp.block(b);
+            uint32_t m[4];
+            bool valid[4];
+            mz_masks<K, MODE == kMaskPass>(sh, t, seq, mask, base + p0 + dev::kMzBlock * b, lane, bLo, bHi, m, valid);
+            if constexpr (MODE == kMaskPass) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const uint32_t q = dev::kMzBlock * b + 32 * i + lane;
+                    uint16_t *to = masks + s * spanLen + q;
+                    if (q < n && (firstPass || m[i]))
+                        *to = (uint16_t)(firstPass ? m[i] : (*to | m[i]));
+                }
+            } else {
+                fold.push(m, valid, lane, (int)K);
+            }
+        }
+        if (MODE != kMaskPass && lane < nSamples)
+            out[(uint64_t)lane * nSpans + s] = seg_of(fold.acc);
     }
 }
 
@@ -383,6 +428,15 @@ int sm_count()
 int grid_for(uint64_t n)
 {
     return (int)std::max<uint64_t>(1, std::min<uint64_t>((n + 255) / 256, (uint64_t)sm_count() * 16));
+}
+
+// Calls f with a minimizer-line joint table's k as a compile-time constant.
+template <uint32_t K = 16, typename F> void with_pm_k(uint32_t k, F &&f)
+{
+    if (k == K)
+        f(std::integral_constant<uint32_t, K>{});
+    else if constexpr (K < 27)
+        with_pm_k<K + 1>(k, f);
 }
 
 // Expected fraction of keys beyond a bucket's kSlots slots when the keys per
@@ -549,9 +603,10 @@ static ibs_status panel_add_device_codes(ibs_panel_table *p, const uint64_t *dCo
     // keys go in chunks, so the build's scratch stays small next to the table
     const uint64_t chunk = std::max<uint64_t>(1, std::min<uint64_t>(n, kBuildChunk));
     uint64_t *pending = nullptr, *failed = nullptr;
-    IBS_CUDA(cudaMalloc(&pending, chunk * 8), "panel pending alloc");
+    const uint64_t places = p->geom.format == FMT_PANEL_MZ ? 2 : 1; // most places a key has
+    IBS_CUDA(cudaMalloc(&pending, chunk * places * 8), "panel pending alloc");
     std::unique_ptr<uint64_t, cudaError_t (*)(void *)> g1(pending, cudaFree);
-    IBS_CUDA(cudaMalloc(&failed, chunk * 8), "panel pending alloc");
+    IBS_CUDA(cudaMalloc(&failed, chunk * places * 8), "panel pending alloc");
     std::unique_ptr<uint64_t, cudaError_t (*)(void *)> g2(failed, cudaFree);
     unsigned long long *cnt = p->dCounters; // [0] pending, [2] failed
     for (uint64_t c0 = 0; c0 < n; c0 += chunk) {
@@ -734,33 +789,34 @@ static ibs_status panel_plan(ibs_panel_table *p, const ibs_reference *ref, uint3
 
 // The span kernel's launches of one scan: one launch, or one per
 // bucket-range pass and a statistics launch.
-template <int NB, bool PM>
-static ibs_status enqueue_spans(ibs_panel_table *p, const ibs_reference *ref, uint32_t passes, int grid,
-                                cudaStream_t st)
+template <int NB>
+static ibs_status enqueue_spans(ibs_panel_table *p, const ibs_reference *ref, uint32_t passes, cudaStream_t st)
 {
     const ScanPlan &pl = p->plan;
-    if (passes <= 1) {
+    const int grid = sm_count() * (int)tuning().panel_ctas_per_sm;
+    const uint64_t nb = p->geom.nBuckets;
+    auto go = [&](auto kernel, uint64_t bLo, uint64_t bHi, bool first) -> ibs_status {
         IBS_CUDA(cudaMemsetAsync(p->dCounters + 1, 0, 8, st), "panel work reset");
-        k_panel_spans<NB, kScan, PM><<<grid, 256, 0, st>>>(p->view(), ref->dSeq, ref->dMask, pl.dWin, pl.dSpan0,
-                                                       (uint32_t)pl.nWin, pl.nSpans, pl.spanLen, p->nSamples,
-                                                       p->dCounters + 1, p->dSpans, nullptr, 0, 0, false);
+        kernel<<<grid, 256, 0, st>>>(p->view(), ref->dSeq, ref->dMask, pl.dWin, pl.dSpan0, (uint32_t)pl.nWin, pl.nSpans,
+                                     pl.spanLen, p->nSamples, p->dCounters + 1, p->dSpans, p->dMasks, bLo, bHi, first);
         IBS_LAUNCHED();
         return IBS_OK;
+    };
+    ibs_status s = IBS_OK;
+    if (passes <= 1) {
+        if (p->geom.format != FMT_PANEL_MZ)
+            return go(k_panel_spans<NB, kScan>, 0, 0, false);
+        with_pm_k(p->geom.k, [&](auto K) { s = go(k_panel_spans_mz<K.value, kScan>, 0, 0, false); });
+        return s;
     }
-    const uint64_t nb = p->geom.nBuckets;
-    for (uint32_t i = 0; i < passes; ++i) {
-        IBS_CUDA(cudaMemsetAsync(p->dCounters + 1, 0, 8, st), "panel work reset");
-        k_panel_spans<NB, kMaskPass, PM><<<grid, 256, 0, st>>>(
-            p->view(), ref->dSeq, ref->dMask, pl.dWin, pl.dSpan0, (uint32_t)pl.nWin, pl.nSpans, pl.spanLen,
-            p->nSamples, p->dCounters + 1, p->dSpans, p->dMasks, nb * i / passes, nb * (i + 1) / passes, i == 0);
-        IBS_LAUNCHED();
+    for (uint32_t i = 0; i < passes && s == IBS_OK; ++i) {
+        const uint64_t bLo = nb * i / passes, bHi = nb * (i + 1) / passes;
+        if (p->geom.format != FMT_PANEL_MZ)
+            s = go(k_panel_spans<NB, kMaskPass>, bLo, bHi, i == 0);
+        else
+            with_pm_k(p->geom.k, [&](auto K) { s = go(k_panel_spans_mz<K.value, kMaskPass>, bLo, bHi, i == 0); });
     }
-    IBS_CUDA(cudaMemsetAsync(p->dCounters + 1, 0, 8, st), "panel work reset");
-    k_panel_spans<NB, kStats, PM><<<grid, 256, 0, st>>>(p->view(), ref->dSeq, ref->dMask, pl.dWin, pl.dSpan0,
-                                                    (uint32_t)pl.nWin, pl.nSpans, pl.spanLen, p->nSamples,
-                                                    p->dCounters + 1, p->dSpans, p->dMasks, 0, 0, false);
-    IBS_LAUNCHED();
-    return IBS_OK;
+    return s == IBS_OK ? go(k_panel_spans<NB, kStats>, 0, 0, false) : s;
 }
 
 static ibs_status panel_enqueue(ibs_panel_table *p, const ibs_reference *ref, ibs_window *rowsDev,
@@ -769,14 +825,8 @@ static ibs_status panel_enqueue(ibs_panel_table *p, const ibs_reference *ref, ib
     const ScanPlan &pl = p->plan;
     const uint32_t passes = pass_count(p);
     if (pl.nSpans) {
-        const ibs_tuning tu = tuning();
-        const int grid = sm_count() * (int)tu.panel_ctas_per_sm;
-        const bool pm = p->geom.format == FMT_PANEL_MZ;
-        const ibs_status s = tu.panel_blocks_in_flight == 2
-                                 ? (pm ? enqueue_spans<2, true>(p, ref, passes, grid, st)
-                                       : enqueue_spans<2, false>(p, ref, passes, grid, st))
-                                 : (pm ? enqueue_spans<4, true>(p, ref, passes, grid, st)
-                                       : enqueue_spans<4, false>(p, ref, passes, grid, st));
+        const ibs_status s = tuning().panel_blocks_in_flight == 2 ? enqueue_spans<2>(p, ref, passes, st)
+                                                                  : enqueue_spans<4>(p, ref, passes, st);
         if (s != IBS_OK)
             return s;
     }

@@ -44,7 +44,7 @@ using dev::canonical_at;
 
 // Feeds NB consecutive 32-position blocks' ballots to the span fold.
 template <int NB>
-__device__ __forceinline__ void fold_blocks(dev::LaneFold &fold, const uint32_t (&V)[NB], const uint32_t (&H)[NB],
+__device__ __forceinline__ void fold_blocks(dev::LaneFold<> &fold, const uint32_t (&V)[NB], const uint32_t (&H)[NB],
                                             uint32_t lane, int k)
 {
 #pragma unroll
@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(512) k_scan_spans(TableView t, const uint64_t 
         const uint32_t nPos = win[w].nPos;
         const uint32_t p0 = (uint32_t)(s - __ldg(span0 + w)) * spanLen;
         const uint32_t p1 = min(p0 + spanLen, nPos);
-        dev::LaneFold fold;
+        dev::LaneFold<> fold;
         for (uint32_t p = p0; p < p1; p += 32 * NB) {
             uint4 v0[NB], v1[NB];
             uint64_t code[NB], fp[NB];
@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(256) k_scan_spans_wide(wide::View t, const uin
         const uint32_t nPos = win[w].nPos;
         const uint32_t p0 = (uint32_t)(s - __ldg(span0 + w)) * spanLen;
         const uint32_t p1 = min(p0 + spanLen, nPos);
-        dev::LaneFold fold;
+        dev::LaneFold<> fold;
         for (uint32_t p = p0; p < p1; p += 32) {
             const uint32_t q = p + lane;
             const bool inSpan = q < p1;
@@ -178,31 +178,31 @@ __global__ void __launch_bounds__(256) k_scan_spans_wide(wide::View t, const uin
 }
 
 // The scan over a minimizer-line table (formats MZ8 and MZ6): one warp per
-// span, the span's statistics from mz_span_stats (mz_scan.cuh). K > 0 fixes
-// k at compile time (the shifts and masks fold); K = 0 reads it from the
-// table. SEC is the sector layout: FMT_B8X32 (format MZ8) or FMT_B6X40
-// (format MZ6).
-template <int NB, uint32_t K, uint32_t SEC>
-__global__ void __launch_bounds__(512) k_scan_spans_mz(TableView t, const uint64_t *__restrict__ seq,
-                                                       const uint64_t *__restrict__ mask,
-                                                       const WinDesc *__restrict__ win,
-                                                       const uint32_t *__restrict__ span0,
-                                                       uint32_t nWin, uint64_t s0, uint64_t s1,
-                                                       uint32_t spanLen, SegStats *__restrict__ out)
+// span, the span's statistics from mz_span_stats (mz_scan.cuh). K is the
+// table's k: every shift and mask of the locator is a compile-time amount
+// (a run-time k ran at 77 G positions/s where k = 25 had 111). SEC is the
+// sector layout: FMT_B8X32 (format MZ8) or FMT_B6X40 (format MZ6).
+constexpr int kMzThreads = 256;
+template <uint32_t K, uint32_t SEC>
+__global__ void __launch_bounds__(kMzThreads, 3) k_scan_spans_mz(const __grid_constant__ TableView t, const uint64_t *__restrict__ seq,
+                                                              const uint64_t *__restrict__ mask,
+                                                              const WinDesc *__restrict__ win,
+                                                              const uint32_t *__restrict__ span0,
+                                                              uint32_t nWin, uint64_t s0, uint64_t s1,
+                                                              uint32_t spanLen, SegStats *__restrict__ out)
 {
-    const uint32_t lane = threadIdx.x & 31;
+    __shared__ dev::MzShared<SEC> shared[kMzThreads / 32];
+    const uint32_t lane = dev::lane_id();
     const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
     const uint64_t nWarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    const uint32_t k = K ? K : t.g.k;
-    const uint32_t w = mz::w_of(k);
     for (uint64_t s = s0 + warp; s < s1; s += nWarps) {
-        const uint32_t wIdx = window_of_span(span0, nWin, s);
-        const uint64_t base = win[wIdx].base;
-        const uint32_t nPos = win[wIdx].nPos;
-        const uint32_t p0 = (uint32_t)(s - __ldg(span0 + wIdx)) * spanLen;
+        const uint32_t w = window_of_span(span0, nWin, s);
+        const uint64_t base = win[w].base;
+        const uint32_t nPos = win[w].nPos;
+        const uint32_t p0 = (uint32_t)(s - __ldg(span0 + w)) * spanLen;
         const uint32_t p1 = min(p0 + spanLen, nPos);
-        // last position read: the last m-mer start the window's k-mers use
-        const SegStats acc = dev::mz_span_stats<NB, K, SEC>(t, seq, mask, base, p0, p1, nPos - 1 + (w - 1), lane);
+        const SegStats acc = dev::mz_span_stats<K, SEC>(&shared[threadIdx.x >> 5], t, seq, mask, base + p0, p1 - p0,
+                                                        base + nPos - 1 + (K - 1), lane);
         if (lane == 0)
             out[s] = acc;
     }
@@ -285,25 +285,23 @@ void plan_windows(ScanPlan &p, const std::vector<uint64_t> &lens,
     p.nSpans = spans;
 }
 
-template <uint32_t FMT, int NB>
-static void launch_nb(const ibs_table *t, const uint64_t *dSeq, const uint64_t *dMask, const ScanPlan &p,
-                      uint64_t s0, uint64_t s1, SegStats *dSpans, cudaStream_t st, int grid, int threads)
+// Minimizer-line tables: one kernel for every k that the format takes.
+template <uint32_t K, uint32_t SEC>
+static void launch_mz(const ibs_table *t, const uint64_t *dSeq, const uint64_t *dMask, const ScanPlan &p, uint64_t s0,
+                      uint64_t s1, SegStats *dSpans, cudaStream_t st)
 {
-    if (FMT == FMT_MZ8 && t->geom.k == 25)
-        k_scan_spans_mz<NB, 25, FMT_B8X32><<<grid, threads, 0, st>>>(t->view(), dSeq, dMask, p.dWin, p.dSpan0,
-                                                                     (uint32_t)p.nWin, s0, s1, p.spanLen, dSpans);
-    else if (FMT == FMT_MZ8)
-        k_scan_spans_mz<NB, 0, FMT_B8X32><<<grid, threads, 0, st>>>(t->view(), dSeq, dMask, p.dWin, p.dSpan0,
-                                                                    (uint32_t)p.nWin, s0, s1, p.spanLen, dSpans);
-    else if (FMT == FMT_MZ6 && t->geom.k == 31)
-        k_scan_spans_mz<NB, 31, FMT_B6X40><<<grid, threads, 0, st>>>(t->view(), dSeq, dMask, p.dWin, p.dSpan0,
-                                                                     (uint32_t)p.nWin, s0, s1, p.spanLen, dSpans);
-    else if (FMT == FMT_MZ6)
-        k_scan_spans_mz<NB, 0, FMT_B6X40><<<grid, threads, 0, st>>>(t->view(), dSeq, dMask, p.dWin, p.dSpan0,
-                                                                    (uint32_t)p.nWin, s0, s1, p.spanLen, dSpans);
-    else
-        k_scan_spans<FMT, NB><<<grid, threads, 0, st>>>(t->view(), dSeq, dMask, p.dWin, p.dSpan0,
-                                                        (uint32_t)p.nWin, s0, s1, p.spanLen, dSpans);
+    if constexpr (SEC == FMT_B8X32 ? K >= 16 && K <= 27 : K >= 16 && K <= 31) {
+        if (t->geom.k != K) {
+            launch_mz<K + 1, SEC>(t, dSeq, dMask, p, s0, s1, dSpans, st);
+            return;
+        }
+        const uint64_t warpsPerCta = kMzThreads / 32;
+        const uint64_t want = (s1 - s0 + warpsPerCta - 1) / warpsPerCta;
+        const uint64_t cap = (uint64_t)sm_count() * tuning().ctas_per_sm * 2; // ctas_per_sm counts CTAs of 512
+        const int grid = (int)std::max<uint64_t>(1, std::min(want, cap));
+        k_scan_spans_mz<K, SEC><<<grid, kMzThreads, 0, st>>>(t->view(), dSeq, dMask, p.dWin, p.dSpan0, (uint32_t)p.nWin,
+                                                            s0, s1, p.spanLen, dSpans);
+    }
 }
 
 template <uint32_t FMT>
@@ -317,11 +315,15 @@ static void launch_spans_fmt(const ibs_table *t, const uint64_t *dSeq, const uin
     const uint64_t want = (s1 - s0 + warpsPerCta - 1) / warpsPerCta;
     const uint64_t cap = (uint64_t)sm_count() * tu.ctas_per_sm;
     const int grid = (int)std::max<uint64_t>(1, std::min(want, cap));
+    auto go = [&](auto kernel) {
+        kernel<<<grid, threads, 0, st>>>(t->view(), dSeq, dMask, p.dWin, p.dSpan0, (uint32_t)p.nWin, s0, s1, p.spanLen,
+                                         dSpans);
+    };
     switch (tu.blocks_in_flight) {
-    case 1: launch_nb<FMT, 1>(t, dSeq, dMask, p, s0, s1, dSpans, st, grid, threads); break;
-    case 2: launch_nb<FMT, 2>(t, dSeq, dMask, p, s0, s1, dSpans, st, grid, threads); break;
-    case 8: launch_nb<FMT, 8>(t, dSeq, dMask, p, s0, s1, dSpans, st, grid, threads); break;
-    default: launch_nb<FMT, 4>(t, dSeq, dMask, p, s0, s1, dSpans, st, grid, threads); break;
+    case 1: go(k_scan_spans<FMT, 1>); break;
+    case 2: go(k_scan_spans<FMT, 2>); break;
+    case 8: go(k_scan_spans<FMT, 8>); break;
+    default: go(k_scan_spans<FMT, 4>); break;
     }
 }
 
@@ -352,9 +354,9 @@ static ibs_status launch_spans(const ibs_table *t, const uint64_t *dSeq, const u
     else if (t->geom.format == FMT_B8X32)
         launch_spans_fmt<FMT_B8X32>(t, dSeq, dMask, p, s0, s1, dSpans, st);
     else if (t->geom.format == FMT_MZ8)
-        launch_spans_fmt<FMT_MZ8>(t, dSeq, dMask, p, s0, s1, dSpans, st);
+        launch_mz<16, FMT_B8X32>(t, dSeq, dMask, p, s0, s1, dSpans, st);
     else if (t->geom.format == FMT_MZ6)
-        launch_spans_fmt<FMT_MZ6>(t, dSeq, dMask, p, s0, s1, dSpans, st);
+        launch_mz<16, FMT_B6X40>(t, dSeq, dMask, p, s0, s1, dSpans, st);
     else
         launch_spans_fmt<FMT_B6X40>(t, dSeq, dMask, p, s0, s1, dSpans, st);
     IBS_LAUNCHED();

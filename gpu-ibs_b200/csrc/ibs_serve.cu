@@ -76,31 +76,35 @@ struct FinItem {
 // positions [p0, p1) of its window goes to sums[it.out]. Minimizer-line
 // tables (MZ8, MZ6) take the window scan's minimizer path
 // (dev::mz_span_stats), the hash-bucket tables one bucket load per
-// position. K > 0 is the server's k fixed at compile time (0: read from the
-// table).
+// position. K > 0 is the server's k fixed at compile time, for every k that
+// a minimizer table can have; K = 0 is any other k, read from the table.
+using MzStorage = dev::MzShared<FMT_B6X40>; // a warp's shared memory, large enough for either layout
 template <int NB, uint32_t K>
 __device__ __forceinline__ void serve_single_item(const WorkItem &it, const TableView &t,
                                                   const uint64_t *__restrict__ seq,
                                                   const uint64_t *__restrict__ mask, SegStats *__restrict__ sums,
-                                                  uint32_t lane)
+                                                  MzStorage *shared, uint32_t lane)
 {
-    if (is_mz(t.g.format)) {
-        // the span's m-mer reads stop at its last position's last m-mer,
-        // inside the window's bases
-        const uint32_t lastM = it.p1 - 1 + (mz::w_of(K ? K : t.g.k) - 1);
-        const SegStats acc =
-            t.g.format == FMT_MZ8
-                ? dev::mz_span_stats<NB, K, FMT_B8X32>(t, seq, mask, it.base, it.p0, it.p1, lastM, lane)
-                : dev::mz_span_stats<NB, K, FMT_B6X40>(t, seq, mask, it.base, it.p0, it.p1, lastM, lane);
-        if (lane == 0)
-            sums[it.out] = acc;
-        return;
+    if constexpr (K >= 16 && K <= 31) {
+        if (is_mz(t.g.format)) {
+            const uint64_t first = it.base + it.p0, lastBase = it.base + it.p1 - 1 + (K - 1);
+            SegStats acc = seg_empty();
+            if (K <= 27 && t.g.format == FMT_MZ8)
+                acc = dev::mz_span_stats<K <= 27 ? K : 27, FMT_B8X32>(
+                    reinterpret_cast<dev::MzShared<FMT_B8X32> *>(shared), t, seq, mask, first, it.p1 - it.p0, lastBase,
+                    lane);
+            else
+                acc = dev::mz_span_stats<K, FMT_B6X40>(shared, t, seq, mask, first, it.p1 - it.p0, lastBase, lane);
+            if (lane == 0)
+                sums[it.out] = acc;
+            return;
+        }
     }
     const uint32_t k = t.g.k;
     const uint64_t kmask = key_mask(2 * k);
     const uint64_t kbits = (1ull << k) - 1;
     const bool b8 = t.g.format == FMT_B8X32;
-    dev::LaneFold fold;
+    dev::LaneFold<> fold;
     for (uint32_t p = it.p0; p < it.p1; p += 32 * NB) {
         uint4 v0[NB], v1[NB];
         uint64_t code[NB], fp[NB];
@@ -170,32 +174,54 @@ __device__ __forceinline__ void fold_run_into(SegStats &acc, uint32_t v, uint32_
 // instead: lane i keeps block i of every 32 and the run is summarised at
 // once, where the per-sample serial block summaries would leave 31 lanes
 // idle. K > 0 is the server's k, which every table of the server has (the
-// server refuses a table of another k): the minimizer window and masks are
-// then compile-time, and the minimizer-line layout is pruned where k rules
-// it out.
-template <int NB, uint32_t K = 0>
+// server refuses a table of another k), for every k that minimizer-line
+// tables can have; those are located 128 positions at a time (mz_scan.cuh).
+template <int NB, uint32_t K>
 __device__ __forceinline__ void serve_joint_item(const WorkItem &it, const panel::View &t,
                                                  const uint64_t *__restrict__ seq,
                                                  const uint64_t *__restrict__ mask, SegStats *__restrict__ sums,
-                                                 uint32_t lane)
+                                                 MzStorage *shared, uint32_t lane)
 {
-    const uint32_t k = K ? K : t.g.k;
-    const uint64_t kmask = key_mask(2 * k);
-    const uint64_t kbits = (1ull << k) - 1;
     const uint32_t want = it.mask & 0xffffu;
     const bool one = (want & (want - 1u)) == 0u; // warp-uniform
     const uint32_t j0 = __ffs(want) - 1;
-    // minimizer-line joint tables (PM) locate a k-mer through its minimizer:
-    // m-mers read one block ahead, up to the span's last position's last
-    // m-mer (inside the window's bases); that layout exists only for
-    // 16 <= k <= 27
-    constexpr bool kPmPossible = K == 0 || (K >= 16 && K <= 27);
-    const bool pm = kPmPossible && t.g.format == FMT_PANEL_MZ;
-    const uint32_t w = pm ? mz::w_of(k) : 1, m = pm ? mz::m_of(k) : 0;
-    const uint32_t lastM = it.p1 - 1 + (w - 1);
-    dev::MzPos next;
-    if (pm)
-        next = dev::mz_pos(seq, mask, it.base + min(it.p0 + lane, lastM), k, m);
+    const uint32_t rank = __popc(want & ((1u << lane) - 1u));
+    if constexpr (K >= 16 && K <= 27) {
+        if (t.g.format == FMT_PANEL_MZ) {
+            auto *sh = reinterpret_cast<dev::MzShared<FMT_B8X32> *>(shared);
+            const uint64_t first = it.base + it.p0;
+            dev::MzWarp<K, FMT_B8X32> warp(sh, t.g, seq, mask, first, it.p1 - it.p0, it.base + it.p1 - 1 + (K - 1),
+                                           lane);
+            dev::LaneFold<true> lone;
+            panel::JointFold fold(lane);
+            warp.start();
+            for (int b = warp.blocks() - 1; b >= 0; --b) {
+                warp.block(b);
+                uint32_t m[4];
+                bool valid[4];
+                panel::mz_masks<K, false>(sh, t, seq, mask, first + dev::kMzBlock * b, lane, 0, 0, m, valid);
+                if (!one) {
+                    fold.push(m, valid, lane, (int)K);
+                    continue;
+                }
+#pragma unroll
+                for (int i = 3; i >= 0; --i)
+                    lone.push(__ballot_sync(dev::FULL_MASK, valid[i]), __ballot_sync(dev::FULL_MASK, (m[i] >> j0) & 1u),
+                              lane, (int)K);
+            }
+            if (one) {
+                const SegStats acc = lone.finish((int)K);
+                if (lane == 0)
+                    sums[it.out] = acc;
+            } else if (lane < 16 && ((want >> lane) & 1u)) {
+                sums[it.out + rank] = seg_of(fold.acc);
+            }
+            return;
+        }
+    }
+    const uint32_t k = K ? K : t.g.k;
+    const uint64_t kmask = key_mask(2 * k);
+    const uint64_t kbits = (1ull << k) - 1;
     SegStats acc = seg_empty();
     uint32_t fv = 0, fh = 0; // one sample: this lane's block of the current run
     for (uint32_t p = it.p0; p < it.p1; p += 32 * NB) {
@@ -203,56 +229,32 @@ __device__ __forceinline__ void serve_joint_item(const WorkItem &it, const panel
         uint64_t code[NB], rr[NB];
         uint32_t fp[NB];
         bool valid[NB];
-        if (pm) {
-            dev::MzPos ps[NB + 1];
-            ps[0] = next;
 #pragma unroll
-            for (int b = 1; b <= NB; ++b)
-                ps[b] = dev::mz_pos(seq, mask, it.base + min(p + 32 * b + lane, lastM), k, m);
-            next = ps[NB];
-#pragma unroll
-            for (int b = 0; b < NB; ++b) {
-                valid[b] = p + 32 * b + lane < it.p1 && ps[b].acgt;
-                uint64_t slot;
-                dev::mz_locate_lane<true>(ps[b], ps[b + 1], lane, k, w, t.g.nBuckets, t.g.fpBits, rr[b], slot);
-                fp[b] = (uint32_t)slot;
-                code[b] = ps[b].code;
-            }
-        } else {
-#pragma unroll
-            for (int b = 0; b < NB; ++b) {
-                const uint32_t q = p + 32 * b + lane;
-                const bool in = q < it.p1;
-                const uint64_t G = it.base + (in ? q : it.p0);
-                bool acgt;
-                code[b] = dev::canonical_at(seq, mask, G, k, kmask, kbits, acgt);
-                valid[b] = in && acgt;
-                const uint64_t h = perm_hash(code[b], t.g.bits);
-                rr[b] = bucket_of(h, t.g);
-                fp[b] = (uint32_t)fp_of(h, t.g);
-            }
+        for (int b = 0; b < NB; ++b) {
+            const uint32_t q = p + 32 * b + lane;
+            const bool in = q < it.p1;
+            const uint64_t G = it.base + (in ? q : it.p0);
+            bool acgt;
+            code[b] = dev::canonical_at(seq, mask, G, k, kmask, kbits, acgt);
+            valid[b] = in && acgt;
+            const uint64_t h = perm_hash(code[b], t.g.bits);
+            rr[b] = bucket_of(h, t.g);
+            fp[b] = (uint32_t)fp_of(h, t.g);
         }
 #pragma unroll
         for (int b = 0; b < NB; ++b) {
-            if (valid[b]) {
-                v0[b] = __ldg(t.buckets + 2 * rr[b]);
-                v1[b] = __ldg(t.buckets + 2 * rr[b] + 1);
-            } else {
-                v0[b] = make_uint4(0, 0, 0, 0);
-                v1[b] = make_uint4(0, 0, 0, 0);
-            }
+            v0[b] = make_uint4(0, 0, 0, 0);
+            v1[b] = make_uint4(0, 0, 0, 0);
+            if (valid[b])
+                load_sector(t.buckets + 2 * rr[b], v0[b], v1[b]);
         }
 #pragma unroll
         for (int b = 0; b < NB; ++b) {
             uint32_t m = 0;
             if (valid[b]) {
-                if (pm) {
-                    m = panel::pm_mask(t, v0[b], v1[b], rr[b], fp[b], code[b]);
-                } else {
-                    m = panel::bucket_mask(v0[b], v1[b], fp[b]);
-                    if (m & 0x80000000u)
-                        m = panel::stash_mask(t, code[b]);
-                }
+                m = panel::bucket_mask(v0[b], v1[b], fp[b]);
+                if (m & 0x80000000u)
+                    m = panel::stash_mask(t, code[b]);
             }
             const uint32_t V = __ballot_sync(dev::FULL_MASK, valid[b]);
             if (one) {
@@ -288,7 +290,7 @@ __device__ __forceinline__ void serve_joint_item(const WorkItem &it, const panel
         return;
     }
     if ((want >> lane) & 1u)
-        sums[it.out + __popc(want & ((1u << lane) - 1u))] = acc;
+        sums[it.out + rank] = acc;
 }
 
 // One (request, window) row from the window's span summaries.
@@ -320,12 +322,13 @@ __global__ void __launch_bounds__(256, 4) k_serve_single(const TableView *__rest
                                                          const uint64_t *__restrict__ mask,
                                                          SegStats *__restrict__ sums)
 {
+    __shared__ MzStorage shared[8];
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
     const uint64_t nWarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
     for (uint64_t i = warp; i < nItems; i += nWarps) {
         const WorkItem it = items[i];
-        serve_single_item<NB, K>(it, views[it.view], seq, mask, sums, lane);
+        serve_single_item<NB, K>(it, views[it.view], seq, mask, sums, &shared[threadIdx.x >> 5], lane);
     }
 }
 
@@ -336,12 +339,13 @@ __global__ void __launch_bounds__(256) k_serve_joint(const panel::View *__restri
                                                      const uint64_t *__restrict__ mask,
                                                      SegStats *__restrict__ sums)
 {
+    __shared__ MzStorage shared[8];
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
     const uint64_t nWarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
     for (uint64_t i = warp; i < nItems; i += nWarps) {
         const WorkItem it = items[i];
-        serve_joint_item<NB, K>(it, views[it.view], seq, mask, sums, lane);
+        serve_joint_item<NB, K>(it, views[it.view], seq, mask, sums, &shared[threadIdx.x >> 5], lane);
     }
 }
 
@@ -492,6 +496,7 @@ __global__ void __launch_bounds__(256, 3) k_serve_persistent(const Ctrl *ctrl, S
                                                              const uint64_t *__restrict__ mask, int k,
                                                              ibs_window *rows, uint64_t idleNs, uint64_t waitNs)
 {
+    __shared__ MzStorage shared[8];
     const uint32_t lane = threadIdx.x & 31;
     // this warp's copy of the batch it worked on last
     uint64_t dT0 = 0, dEnd = 0;
@@ -611,10 +616,10 @@ __global__ void __launch_bounds__(256, 3) k_serve_persistent(const Ctrl *ctrl, S
         if (local < nScan) {
             if (local < d.nSingle) {
                 const WorkItem it = d.single[local];
-                serve_single_item<NB, K>(it, d.sv[it.view], seq, mask, d.sums, lane);
+                serve_single_item<NB, K>(it, d.sv[it.view], seq, mask, d.sums, &shared[threadIdx.x >> 5], lane);
             } else {
                 const WorkItem it = d.joint[local - d.nSingle];
-                serve_joint_item<NB, K>(it, d.jv[it.view], seq, mask, d.sums, lane);
+                serve_joint_item<NB, K>(it, d.jv[it.view], seq, mask, d.sums, &shared[threadIdx.x >> 5], lane);
             }
             __threadfence(); // every lane's summaries are visible before the count
             __syncwarp();
@@ -678,6 +683,18 @@ __global__ void __launch_bounds__(256, 3) k_serve_persistent(const Ctrl *ctrl, S
             }
         }
     }
+}
+
+// Calls f with the server's k as a compile-time constant: every k that a
+// minimizer table can have, else 0.
+template <uint32_t K = 16, typename F> void with_k(uint32_t k, F &&f)
+{
+    if (k < 16 || K > 31)
+        f(std::integral_constant<uint32_t, 0>{});
+    else if (k == K)
+        f(std::integral_constant<uint32_t, K <= 31 ? K : 0>{});
+    else if constexpr (K <= 31)
+        with_k<K + 1>(k, f);
 }
 
 // First-fit allocator of [offset, offset+size) ranges of a pool.
@@ -1003,18 +1020,11 @@ bool start_kernel(ibs_server *s)
     std::atomic_thread_fence(std::memory_order_seq_cst);
     cudaError_t e = cudaMemsetAsync(s->ds, 0, sizeof(DevState), s->comp);
     if (e == cudaSuccess) {
-        if (s->k == 25)
-            k_serve_persistent<kServeNB, 25><<<s->persistentGrid, 256, 0, s->comp>>>(
+        with_k(s->k, [&](auto K) {
+            k_serve_persistent<kServeNB, K.value><<<s->persistentGrid, 256, 0, s->comp>>>(
                 s->dCtrl, s->dStatus, s->ds, s->ref->dSeq, s->ref->dMask, (int)s->k, s->dRowsMapped, s->idleNs,
                 s->waitNs);
-        else if (s->k == 31)
-            k_serve_persistent<kServeNB, 31><<<s->persistentGrid, 256, 0, s->comp>>>(
-                s->dCtrl, s->dStatus, s->ds, s->ref->dSeq, s->ref->dMask, (int)s->k, s->dRowsMapped, s->idleNs,
-                s->waitNs);
-        else
-            k_serve_persistent<kServeNB, 0><<<s->persistentGrid, 256, 0, s->comp>>>(
-                s->dCtrl, s->dStatus, s->ds, s->ref->dSeq, s->ref->dMask, (int)s->k, s->dRowsMapped, s->idleNs,
-                s->waitNs);
+        });
         IBS_LAUNCHED();
         e = cudaGetLastError();
     }
@@ -1459,28 +1469,18 @@ bool iterate(ibs_server *s)
     cudaEventRecord(L.start, st);
     if (nSingle) {
         const int grid = (int)std::min<uint64_t>((nSingle + 7) / 8, (uint64_t)s->sms * 8);
-        if (s->k == 25)
-            k_serve_single<kServeNB, 25><<<grid, 256, 0, st>>>(L.dSV, L.dSingle, nSingle, s->ref->dSeq,
-                                                          s->ref->dMask, L.dSums);
-        else if (s->k == 31)
-            k_serve_single<kServeNB, 31><<<grid, 256, 0, st>>>(L.dSV, L.dSingle, nSingle, s->ref->dSeq,
-                                                          s->ref->dMask, L.dSums);
-        else
-            k_serve_single<kServeNB, 0><<<grid, 256, 0, st>>>(L.dSV, L.dSingle, nSingle, s->ref->dSeq,
-                                                         s->ref->dMask, L.dSums);
+        with_k(s->k, [&](auto K) {
+            k_serve_single<kServeNB, K.value><<<grid, 256, 0, st>>>(L.dSV, L.dSingle, nSingle, s->ref->dSeq,
+                                                                    s->ref->dMask, L.dSums);
+        });
         IBS_LAUNCHED();
     }
     if (nJoint) {
         const int grid = (int)std::min<uint64_t>((nJoint + 7) / 8, (uint64_t)s->sms * 8);
-        if (s->k == 25)
-            k_serve_joint<kNB, 25><<<grid, 256, 0, st>>>(L.dJV, L.dJoint, nJoint, s->ref->dSeq, s->ref->dMask,
-                                                         L.dSums);
-        else if (s->k == 31)
-            k_serve_joint<kNB, 31><<<grid, 256, 0, st>>>(L.dJV, L.dJoint, nJoint, s->ref->dSeq, s->ref->dMask,
-                                                         L.dSums);
-        else
-            k_serve_joint<kNB, 0><<<grid, 256, 0, st>>>(L.dJV, L.dJoint, nJoint, s->ref->dSeq, s->ref->dMask,
-                                                        L.dSums);
+        with_k(s->k, [&](auto K) {
+            k_serve_joint<kNB, K.value><<<grid, 256, 0, st>>>(L.dJV, L.dJoint, nJoint, s->ref->dSeq, s->ref->dMask,
+                                                              L.dSums);
+        });
         IBS_LAUNCHED();
     }
     if (nFin) {
@@ -1653,12 +1653,9 @@ extern "C" ibs_status ibs_server_create(ibs_reference *ref, uint32_t W, uint32_t
         IBS_CUDA(cudaMalloc(&s->ds, sizeof(DevState)), "persistent state");
         IBS_CUDA(cudaEventCreateWithFlags(&s->kernelEnd, cudaEventDisableTiming), "event create");
         int perSm = 0;
-        if (s->k == 25)
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_serve_persistent<kServeNB, 25>, 256, 0);
-        else if (s->k == 31)
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_serve_persistent<kServeNB, 31>, 256, 0);
-        else
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_serve_persistent<kServeNB, 0>, 256, 0);
+        with_k(s->k, [&](auto K) {
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_serve_persistent<kServeNB, K.value>, 256, 0);
+        });
         s->persistentGrid = s->sms * std::max(1, perSm);
     }
     for (auto &L : s->launches) {

@@ -63,7 +63,7 @@ static TableGeom choose_geometry(uint64_t nKeys, uint32_t k, const ibs_table_opt
     const bool tunedMz = tuning().table_format == FMT_MZ8;
     // minimum line count of a minimizer table: its slot values must fit 31
     // bits (B8x32 sectors, k <= 27) or 40 bits (B6x40 sectors, k <= 31)
-    auto mzMinLog2 = [&](uint32_t f) { return (int)(2 * k) - (f == FMT_MZ8 ? 27 : 36); };
+    auto mzMinLog2 = [&](uint32_t f) { return (int)(2 * k) - (f == FMT_MZ8 ? 28 : 37); };
     if (fmt == 0 && tunedMz && k >= 16 && k <= 31) {
         // the tuned default, where the minimizer layout applies and its
         // minimum line count does not oversize the table
@@ -121,92 +121,17 @@ static TableGeom choose_geometry(uint64_t nKeys, uint32_t k, const ibs_table_opt
 // ---------------------------------------------------------------------------
 // build kernels
 // ---------------------------------------------------------------------------
-// Bucket and stored fingerprint of a key in either table family.
-__device__ __forceinline__ void locate_key(uint64_t code, const TableGeom &g, uint64_t &r, uint64_t &fp)
+// Buckets and stored fingerprints of a key in either table family; returns how
+// many places it has (a minimizer table files a k-mer whose leftmost and
+// rightmost minimizers differ under both: mz::placements).
+__device__ __forceinline__ uint32_t locate_key(uint64_t code, const TableGeom &g, uint64_t r[2], uint64_t fp[2])
 {
-    if (is_mz(g.format)) {
-        mz::locate(code, g, r, fp);
-        return;
-    }
+    if (is_mz(g.format))
+        return mz::placements(code, g, r, fp);
     const uint64_t h = perm_hash(code, g.bits);
-    r = bucket_of(h, g);
-    fp = fp_of(h, g);
-}
-
-__global__ void k_count(const uint64_t *__restrict__ codes, uint64_t n, TableGeom g,
-                        uint32_t *__restrict__ cnt)
-{
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
-         i += (uint64_t)gridDim.x * blockDim.x) {
-        uint64_t r, fp;
-        locate_key(codes[i], g, r, fp);
-        atomicAdd(cnt + r, 1u);
-    }
-}
-
-// Marks overflowing buckets, records B6x40 counts, sums the keys that go to
-// the stash and resets the counters for the placement pass.
-__global__ void k_mark(uint32_t *__restrict__ cnt, uint64_t nb, TableGeom g,
-                       uint32_t *__restrict__ words, unsigned long long *__restrict__ overflowKeys)
-{
-    unsigned long long local = 0;
-    for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < nb;
-         r += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t c = cnt[r];
-        if (g.format == FMT_B8X32) {
-            if (c > 8) {
-                words[r * 8 + 7] = B8_OVERFLOW;
-                local += c - 7;
-            }
-        } else {
-            const uint32_t keep = c > 6 ? 6 : c;
-            const uint32_t flags = c > 6 ? 1u : 0u;
-            if (c > 6)
-                local += c - 6;
-            words[r * 8 + 7] = (words[r * 8 + 7] & 0x0000ffffu) | (keep << 16) | (flags << 24);
-        }
-        cnt[r] = 0;
-    }
-    for (int o = 16; o; o >>= 1)
-        local += __shfl_xor_sync(0xffffffffu, local, o);
-    if ((threadIdx.x & 31) == 0 && local)
-        atomicAdd(overflowKeys, local);
-}
-
-// MZ8: marks full sectors pair by pair (sectors 2i and 2i + 1 of a line are
-// partners). A sector with c > 8 keys keeps 7 and sends c - 7 to its
-// partner's free slots (8 - c' when the partner holds c' < 8) and the rest to
-// the stash. Sums the keys leaving their sector (spill) and those reaching
-// the stash, and resets the counters for the placement pass.
-__global__ void k_mark_mz8(uint32_t *__restrict__ cnt, uint64_t nb, uint32_t *__restrict__ words,
-                           unsigned long long *__restrict__ spillKeys, unsigned long long *__restrict__ stashKeys)
-{
-    unsigned long long spill = 0, stash = 0;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; 2 * i < nb;
-         i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t r = 2 * i;
-        const uint32_t c[2] = {cnt[r], cnt[r + 1]};
-        for (int a = 0; a < 2; ++a) {
-            if (c[a] > 8) {
-                const uint32_t extra = c[a] - 7;
-                const uint32_t room = c[a ^ 1] < 8 ? 8 - c[a ^ 1] : 0;
-                words[(r + a) * 8 + 7] = extra > room ? B8_OVERFLOW_STASH : B8_OVERFLOW;
-                spill += extra;
-                stash += extra > room ? extra - room : 0;
-            }
-        }
-        cnt[r] = cnt[r + 1] = 0;
-    }
-    for (int o = 16; o; o >>= 1) {
-        spill += __shfl_xor_sync(0xffffffffu, spill, o);
-        stash += __shfl_xor_sync(0xffffffffu, stash, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-        if (spill)
-            atomicAdd(spillKeys, spill);
-        if (stash)
-            atomicAdd(stashKeys, stash);
-    }
+    r[0] = bucket_of(h, g);
+    fp[0] = fp_of(h, g);
+    return 1;
 }
 
 __device__ __forceinline__ bool stash_insert(uint64_t *stash, uint64_t stashBuckets, uint64_t code)
@@ -225,71 +150,147 @@ __device__ __forceinline__ bool stash_insert(uint64_t *stash, uint64_t stashBuck
     return false;
 }
 
-// Places every key in its bucket; the extra keys of a full bucket go to the
-// stash, or for MZ8 to the spill list (placed by k_spill_mz8 once every
-// sector holds its own keys).
-__global__ void k_place(const uint64_t *__restrict__ codes, uint64_t n, TableGeom g,
-                        uint32_t *__restrict__ cnt, uint32_t *__restrict__ words,
-                        uint64_t *__restrict__ stash, uint64_t *__restrict__ spillList,
-                        unsigned long long *__restrict__ spillN, uint64_t spillCap, int *__restrict__ err)
+// ---- placement ---------------------------------------------------------------
+// Every key takes a free slot of its bucket in one pass over the keys
+// (k_fill): the bucket is read and the slot claimed by a compare-and-swap on
+// the same line, so a key costs one random line. (Counting the keys of every
+// bucket first and placing them in a second pass touched three: 14 ms against
+// 6 for 220M keys.) Keys that find no slot go to a list, and a second, small
+// pass (k_spill) settles those.
+
+// Claims one of 32-bit slots [0, last) of a B8x32 bucket for fp; true when it
+// is there (an equal value there already counts: a duplicate key).
+__device__ __forceinline__ bool claim8(uint32_t *w, uint32_t fp, uint32_t last)
 {
-    uint8_t *bytes = reinterpret_cast<uint8_t *>(words);
+    const uint4 a = __ldcg(reinterpret_cast<const uint4 *>(w)), b = __ldcg(reinterpret_cast<const uint4 *>(w) + 1);
+    const uint32_t v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+    for (uint32_t j = 0; j < 8; ++j) {
+        if (j >= last)
+            break;
+        if (v[j] == fp)
+            return true;
+        if (v[j] == B8_EMPTY) {
+            const uint32_t old = atomicCAS(w + j, B8_EMPTY, fp);
+            if (old == B8_EMPTY || old == fp)
+                return true;
+        }
+    }
+    return false;
+}
+
+// The same for a B6x40 bucket, whose count byte says which slots are taken.
+__device__ __forceinline__ bool claim6(uint32_t *w, uint64_t fp)
+{
+    uint32_t old = __ldcg(w + 7);
+    for (int tries = 0; tries < 1 << 20; ++tries) {
+        const uint32_t s = (old >> 16) & 0xffu;
+        if (s >= 6)
+            return false;
+        const uint32_t seen = atomicCAS(w + 7, old, old + (1u << 16));
+        if (seen == old) {
+            w[s] = (uint32_t)(fp >> 8);
+            // bytes 24 .. 29: two of them share word 7 with the count
+            atomicOr(w + 6 + s / 4, (uint32_t)(fp & 0xff) << (8 * (s & 3)));
+            return true;
+        }
+        old = seen;
+    }
+    return false;
+}
+
+// Slot 7 of a B8x32 bucket stays free in this pass: it becomes a key's when
+// one key is left over, or the marker when there are more.
+__global__ void k_fill(const uint64_t *__restrict__ codes, uint64_t n, TableGeom g, uint32_t *__restrict__ words,
+                       uint64_t *__restrict__ list, unsigned long long *__restrict__ listN, uint64_t listCap)
+{
+    const bool b8 = g.format == FMT_B8X32 || g.format == FMT_MZ8;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
          i += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t code = codes[i];
-        uint64_t r, fp;
-        locate_key(code, g, r, fp);
-        const uint32_t s = atomicAdd(cnt + r, 1u);
-        bool stashed = false;
-        if (g.format == FMT_MZ8) {
-            const uint32_t w7 = words[r * 8 + 7];
-            const uint32_t limit = (w7 == B8_OVERFLOW || w7 == B8_OVERFLOW_STASH) ? 7u : 8u;
-            if (s < limit) {
-                words[r * 8 + s] = (uint32_t)fp;
-            } else {
-                const unsigned long long j = atomicAdd(spillN, 1ull);
-                if (j < spillCap)
-                    spillList[j] = code;
-                else
-                    atomicExch(err, 1);
-            }
-        } else if (g.format == FMT_B8X32) {
-            const uint32_t limit = words[r * 8 + 7] == B8_OVERFLOW ? 7u : 8u;
-            if (s < limit)
-                words[r * 8 + s] = (uint32_t)fp;
-            else
-                stashed = true;
-        } else {
-            if (s < 6) {
-                words[r * 8 + s] = (uint32_t)(fp >> 8);
-                bytes[r * 32 + 24 + s] = (uint8_t)(fp & 0xff);
-            } else
-                stashed = true;
+        uint64_t rr[2], ff[2];
+        const uint32_t places = locate_key(code, g, rr, ff);
+        for (uint32_t a = 0; a < places || a == 0; ++a) {
+            const uint64_t r = a ? rr[1] : rr[0], fp = a ? ff[1] : ff[0];
+            if (places && (b8 ? claim8(words + r * 8, (uint32_t)fp, 7) : claim6(words + r * 8, fp)))
+                continue;
+            const unsigned long long j = atomicAdd(listN, 1ull);
+            if (j < listCap)
+                list[j] = code | (!places ? mz::kNoPlace : a ? mz::kSecondPlace : 0ull);
         }
-        if (stashed && !stash_insert(stash, g.stashBuckets, code))
-            atomicExch(err, 1);
     }
 }
 
-// MZ8 spill pass: each extra key takes the next free slot of its partner
-// sector (after the partner's own keys, all placed by k_place), or the stash
-// once the partner is full. The numbers that land in each place follow from
-// the counts, as k_mark_mz8 recorded them in the sector markers.
-__global__ void k_spill_mz8(const uint64_t *__restrict__ spillList, uint64_t n, TableGeom g,
-                            uint32_t *__restrict__ cnt, uint32_t *__restrict__ words, uint64_t *__restrict__ stash,
-                            int *__restrict__ err)
+// B8x32 sectors: the number of listed keys of each bucket, up to 3, two bits a
+// bucket.
+__global__ void k_count_left(const uint64_t *__restrict__ list, uint64_t n, TableGeom g, uint32_t *__restrict__ left)
 {
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
          i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t code = spillList[i];
-        uint64_t r, fp;
-        locate_key(code, g, r, fp);
-        const uint32_t s = atomicAdd(cnt + (r ^ 1), 1u);
-        if (s < 8)
-            words[(r ^ 1) * 8 + s] = (uint32_t)fp;
-        else if (!stash_insert(stash, g.stashBuckets, code))
-            atomicExch(err, 1);
+        const bool mz = is_mz(g.format);
+        if (mz && (list[i] & mz::kNoPlace))
+            continue;
+        uint64_t rr[2], ff[2];
+        locate_key(mz ? list[i] & ~mz::kSecondPlace : list[i], g, rr, ff);
+        const uint64_t r = mz && (list[i] & mz::kSecondPlace) ? rr[1] : rr[0];
+        // the first key sets the low bit, any further one the high bit
+        const uint32_t one = 1u << (2 * (r & 15));
+        if (atomicOr(left + (r >> 4), one) & one)
+            atomicOr(left + (r >> 4), one << 1);
     }
+}
+
+// Settles the listed keys: a B8x32 bucket's only one takes slot 7; otherwise
+// a minimizer line's go to the line's free slots, the partner sector's first
+// (a sector's slot 7 only where that sector has no listed keys of its own),
+// and what is left, as every listed key of a hash bucket, to the stash list.
+// The home bucket's marker says how far.
+__global__ void k_spill(const uint64_t *__restrict__ list, uint64_t n, TableGeom g, const uint32_t *__restrict__ left,
+                        uint32_t *__restrict__ words, uint64_t *__restrict__ stashList,
+                        unsigned long long *__restrict__ stashN)
+{
+    const bool b8 = g.format == FMT_B8X32 || g.format == FMT_MZ8, mz = is_mz(g.format);
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
+         i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t code = mz ? list[i] & ~(mz::kSecondPlace | mz::kNoPlace) : list[i];
+        if (mz && (list[i] & mz::kNoPlace)) {
+            stashList[atomicAdd(stashN, 1ull)] = code;
+            continue;
+        }
+        uint64_t rr[2], ff[2];
+        locate_key(code, g, rr, ff);
+        const uint32_t a = mz ? (uint32_t)(list[i] >> 63) : 0; // which of its places
+        const uint64_t r = a ? rr[1] : rr[0], fp = a ? ff[1] : ff[0];
+        uint32_t *home = words + r * 8;
+        auto left_of = [&](uint64_t x) { return (left[x >> 4] >> (2 * (x & 15))) & 3u; };
+        if (b8 && left_of(r) == 1u) {
+            home[7] = (uint32_t)fp;
+            continue;
+        }
+        uint32_t reach = 3;
+        for (uint32_t d = 1; d < 4 && mz && reach == 3; ++d) {
+            uint32_t *w = words + (r ^ d) * 8;
+            if (b8 ? claim8(w, (uint32_t)fp, left_of(r ^ d) ? 7 : 8) : claim6(w, fp))
+                reach = d == 1 ? 1 : 2;
+        }
+        if (reach == 3)
+            stashList[atomicAdd(stashN, 1ull)] = code;
+        if (!mz)
+            reach = 1; // hash buckets: the marker (B8_OVERFLOW, flag bit 0) means the stash
+        if (b8)
+            atomicMin(home + 7, 0xffffffffu - reach); // EMPTY, then the markers downwards
+        else
+            atomicOr(home + 7, reach << 24); // 1 | 2 reads as 3: one place more is looked at
+    }
+}
+
+__global__ void k_stash(const uint64_t *__restrict__ list, uint64_t n, uint64_t *__restrict__ stash,
+                        uint64_t stashBuckets, int *__restrict__ err)
+{
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
+         i += (uint64_t)gridDim.x * blockDim.x)
+        if (!stash_insert(stash, stashBuckets, list[i]))
+            atomicExch(err, 1);
 }
 
 // Record r of a .kmc_suf chunk -> canonical code. The LUT bucket j holding
@@ -397,76 +398,75 @@ static ibs_status build_from_device_codes(ibs_table *t, const uint64_t *dCodes, 
     t->nKeys = n;
     TableGeom &g = t->geom;
     const uint64_t nb = g.nBuckets;
+    const bool b8 = g.format == FMT_B8X32 || g.format == FMT_MZ8;
     IBS_CUDA(cudaMalloc(&t->buckets, nb * 32), "table alloc");
     t->deviceBytes = nb * 32;
-    IBS_CUDA(cudaMemset(t->buckets, g.format == FMT_B6X40 || g.format == FMT_MZ6 ? 0x00 : 0xff, nb * 32),
-             "table init");
-    uint32_t *cnt = nullptr;
-    unsigned long long *dOverflow = nullptr; // [0] keys to the stash, [1] MZ8 spill keys, [2] spill list fill
-    uint64_t *spillList = nullptr;
-    int *dErr = nullptr;
-    auto cleanup = [&]() {
-        cudaFree(cnt);
-        cudaFree(dOverflow);
-        cudaFree(spillList);
-        cudaFree(dErr);
-    };
-    cudaError_t e = cudaMalloc(&cnt, nb * 4);
-    if (e == cudaSuccess)
-        e = cudaMalloc(&dOverflow, 3 * 8);
-    if (e == cudaSuccess)
-        e = cudaMalloc(&dErr, sizeof(int));
-    if (e == cudaSuccess)
-        e = cudaMemset(cnt, 0, nb * 4);
-    if (e == cudaSuccess)
-        e = cudaMemset(dOverflow, 0, 3 * 8);
-    if (e == cudaSuccess)
-        e = cudaMemset(dErr, 0, sizeof(int));
-    if (e != cudaSuccess) {
-        cleanup();
-        return cuda_fail(e, "table build scratch");
-    }
-    uint32_t *words = reinterpret_cast<uint32_t *>(t->buckets);
-    k_count<<<grid_for(n, 256), 256>>>(dCodes, n, g, cnt);
-    IBS_LAUNCHED();
-    if (g.format == FMT_MZ8)
-        k_mark_mz8<<<grid_for(nb / 2, 256), 256>>>(cnt, nb, words, dOverflow + 1, dOverflow);
-    else
-        k_mark<<<grid_for(nb, 256), 256>>>(cnt, nb, g, words, dOverflow);
-    IBS_LAUNCHED();
-    unsigned long long counts[2] = {0, 0}; // keys to the stash, MZ8 keys leaving their sector
-    e = cudaMemcpy(counts, dOverflow, 2 * 8, cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess && counts[1])
-        e = cudaMalloc(&spillList, counts[1] * 8);
-    if (e != cudaSuccess) {
-        cleanup();
-        return cuda_fail(e, "table build count");
-    }
-    const unsigned long long overflow = counts[0];
-    t->stashKeys = overflow;
-    if (overflow) {
-        g.stashBuckets = next_pow2((overflow * 2 + 3) / 4);
-        e = cudaMalloc(&t->stash, g.stashBuckets * 32);
-        if (e == cudaSuccess)
-            e = cudaMemset(t->stash, 0xff, g.stashBuckets * 32);
-        if (e != cudaSuccess) {
-            cleanup();
-            return cuda_fail(e, "stash alloc");
+    struct Scratch {
+        unsigned long long *counts = nullptr; // [0] listed keys, [1] keys for the stash, [2] error
+        uint64_t *list = nullptr, *stashList = nullptr;
+        uint32_t *left = nullptr;
+        ~Scratch()
+        {
+            cudaFree(counts);
+            cudaFree(list);
+            cudaFree(stashList);
+            cudaFree(left);
         }
-        t->deviceBytes += g.stashBuckets * 32;
+    } x;
+    IBS_CUDA(cudaMalloc(&x.counts, 3 * 8), "table build scratch");
+    uint32_t *words = reinterpret_cast<uint32_t *>(t->buckets);
+    unsigned long long counts[2] = {0, 0};
+    // about 2% of the keys find no slot at the default loads; a table that
+    // leaves more (a forced load, many duplicates) is filled again with a
+    // list of the size that it then needs and as much again
+    uint64_t listCap = n / 16 + 4096;
+    for (int attempt = 0;; ++attempt) {
+        IBS_CUDA(cudaMalloc(&x.list, listCap * 8), "table build scratch");
+        IBS_CUDA(cudaMemsetAsync(t->buckets, b8 ? 0xff : 0x00, nb * 32, 0), "table init");
+        IBS_CUDA(cudaMemsetAsync(x.counts, 0, 3 * 8, 0), "table build scratch");
+        if (n) {
+            k_fill<<<grid_for(n, 256), 256>>>(dCodes, n, g, words, x.list, x.counts, listCap);
+            IBS_LAUNCHED();
+        }
+        IBS_CUDA(cudaMemcpy(counts, x.counts, 8, cudaMemcpyDeviceToHost), "table build fill");
+        if (counts[0] <= listCap)
+            break;
+        if (attempt == 3) {
+            set_error("table build: the list of keys without a slot keeps growing");
+            return IBS_ERR_CAPACITY;
+        }
+        cudaFree(x.list);
+        x.list = nullptr;
+        listCap = 2 * counts[0];
     }
-    k_place<<<grid_for(n, 256), 256>>>(dCodes, n, g, cnt, words, t->stash, spillList, dOverflow + 2, counts[1],
-                                       dErr);
-    IBS_LAUNCHED();
-    if (counts[1]) {
-        k_spill_mz8<<<grid_for(counts[1], 256), 256>>>(spillList, counts[1], g, cnt, words, t->stash, dErr);
+    t->stashKeys = 0;
+    if (!counts[0])
+        return IBS_OK;
+    const uint64_t listed = counts[0];
+    IBS_CUDA(cudaMalloc(&x.stashList, listed * 8), "table build scratch");
+    if (b8) {
+        const uint64_t leftBytes = (nb + 15) / 16 * 4;
+        IBS_CUDA(cudaMalloc(&x.left, leftBytes), "table build scratch");
+        IBS_CUDA(cudaMemsetAsync(x.left, 0, leftBytes, 0), "table build scratch");
+        k_count_left<<<grid_for(listed, 256), 256>>>(x.list, listed, g, x.left);
         IBS_LAUNCHED();
     }
+    k_spill<<<grid_for(listed, 256), 256>>>(x.list, listed, g, x.left, words, x.stashList, x.counts + 1);
+    IBS_LAUNCHED();
+    IBS_CUDA(cudaMemcpy(counts + 1, x.counts + 1, 8, cudaMemcpyDeviceToHost), "table build spill");
+    t->stashKeys = counts[1];
+    if (!counts[1])
+        return IBS_OK;
+    const uint64_t stashBuckets = next_pow2((counts[1] * 2 + 3) / 4);
+    IBS_CUDA(cudaMalloc(&t->stash, stashBuckets * 32), "stash alloc");
+    g.stashBuckets = stashBuckets;
+    t->deviceBytes += stashBuckets * 32;
+    IBS_CUDA(cudaMemsetAsync(t->stash, 0xff, stashBuckets * 32, 0), "stash alloc");
+    k_stash<<<grid_for(counts[1], 256), 256>>>(x.stashList, counts[1], t->stash, stashBuckets,
+                                               reinterpret_cast<int *>(x.counts + 2));
+    IBS_LAUNCHED();
     int herr = 0;
-    e = cudaMemcpy(&herr, dErr, sizeof(int), cudaMemcpyDeviceToHost);
-    cleanup();
-    if (e != cudaSuccess)
-        return cuda_fail(e, "table build place");
+    IBS_CUDA(cudaMemcpy(&herr, x.counts + 2, sizeof herr, cudaMemcpyDeviceToHost), "table build stash");
     if (herr) {
         set_error("table build: stash full");
         return IBS_ERR_CAPACITY;

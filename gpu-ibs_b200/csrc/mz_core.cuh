@@ -1,31 +1,33 @@
 // Minimizer-bucketed table (format MZ8): the key -> (bucket, slot) map.
 //
-// A canonical k-mer C is filed under its minimizer: among C's w = k - m + 1
-// m-mers (m = k - 6 from k = 22, else 16), the one whose canonical form has
-// the smallest rank key (29 bits derived from the m-mer's line hash, below),
-// ties going to the leftmost in C. Consecutive
-// reference positions mostly share their minimizer (runs of up to w
-// positions), so their probes fall in one place of the table. m grows with k so that a minimizer rarely occurs at
-// two loci of a large genome (4^19 19-mers against 2e9 positions), which
-// would pile two runs into one place.
+// A k-mer is filed under its minimizer: among its w = k - m + 1 m-mers (m =
+// k - 7 from k = 23, else 16), the one whose canonical form has the smallest
+// rank key (27 bits derived from the m-mer's hash, below), ties going to the
+// leftmost (placements() below has what that means on either strand).
+// Consecutive reference positions mostly share their minimizer: the scan
+// touches a new line every (w + 1) / 2 = 4.5 positions on average, and the
+// random lines of a table beyond a few GB come at 36.4 G/s at most on a B200
+// (one 32-byte load each; measured), which bounds the scan. m grows with k so
+// that a minimizer rarely occurs at two loci of a large genome (4^18 18-mers
+// against 2e9 positions), which would pile two runs into one place.
 //
 // The table is an array of 128-byte lines of four 32-byte sectors; a sector
 // is a B8x32 bucket (format MZ8) or a B6x40 bucket (format MZ6). The
-// minimizer picks the line and C itself picks one of its four sectors, so a
+// minimizer picks the line and the slot value one of its four sectors, so a
 // minimizer's k-mers spread over the line and a warp's loads for a run of
 // positions touch one DRAM line.
 //
-// The slot value identifies C exactly inside its line: with g = line_hash(M)
-// (a bijection of the 2m-bit canonical minimizer M), line = the top 32 bits
-// of g scaled to [0, nLines), so the low hbits = 2m - floor(log2(nLines))
-// bits of g single out g, hence M, among the line's interval; C is then M at
-// offset o (< w <= 8), in orientation s (M or its reverse complement), with
-// the other k - m bases around it:
-//   slot = ((o << 1 | s) << 2(k-m) | C-without-the-m-mer) << hbits | (g mod 2^hbits)
-// which has 2k + 4 - floor(log2(nLines)) bits and must fit the sector's slots: 31
-// bits in B8x32 sectors (format MZ8, the sentinels above), nLines >=
-// 2^(2k-27); 40 bits in B6x40 sectors (format MZ6, for k up to 31), nLines
-// >= 2^(2k-36).
+// The slot value identifies the k-mer exactly inside its line: with g =
+// line_hash(M) (a bijection of the 2m-bit canonical minimizer M), line = the
+// top 32 bits of g scaled to [0, nLines), so the low hbits = 2m -
+// floor(log2(nLines)) bits of g single out g, hence M, among the line's
+// interval; the k-mer, on the strand where it holds M itself, is then M at
+// offset o (< w <= 8) with the other k - m bases around it:
+//   slot = (o << 2(k-m) | k-mer-without-the-m-mer) << hbits | (g mod 2^hbits)
+// which has 2k + 3 - floor(log2(nLines)) bits and must fit the sector's slots:
+// 31 bits in B8x32 sectors (format MZ8, the sentinels above), nLines >=
+// 2^(2k-28); 40 bits in B6x40 sectors (format MZ6, for k up to 31), nLines
+// >= 2^(2k-37).
 #pragma once
 
 #include "ibs_core.cuh"
@@ -34,8 +36,11 @@ namespace ibs {
 namespace mz {
 
 constexpr uint32_t kSectorsPerLine = 4;
+// Flags of a key in the builds' lists of keys without a slot (2k <= 62 bits):
+// its second place is meant, or it has none (not canonical).
+constexpr uint64_t kSecondPlace = 1ull << 63, kNoPlace = 1ull << 62;
 
-IBS_HD uint32_t m_of(uint32_t k) { return k >= 22 ? k - 6 : 16; }
+IBS_HD uint32_t m_of(uint32_t k) { return k >= 23 ? k - 7 : 16; }
 IBS_HD uint32_t w_of(uint32_t k) { return k - m_of(k) + 1; }
 
 IBS_HD uint64_t brev64(uint64_t x)
@@ -66,29 +71,42 @@ IBS_HD uint64_t canon_m(uint64_t v, uint32_t m)
     return v < r ? v : r;
 }
 
-// The line hash of a canonical m-mer: a bijection of the 2m-bit values, two
-// multiply-xorshift rounds, so the lines stay uniform over the minimizers.
-IBS_HD uint64_t line_hash(uint64_t canonical, uint32_t m)
+// A canonical m-mer's hash, a bijection of its 2m bits (32 <= 2m <= 50) on two
+// 32-bit words (lo from the m-mer's top 32 bits, hi its 2m - 32 low bits,
+// which stay as they are): the scan computes one per reference position, so
+// it is five instructions; the 64-bit multiply-xorshift rounds it replaces
+// were about 18. Given hi, each step is a bijection of lo.
+struct Mixed {
+    uint32_t lo, hi;
+};
+
+IBS_HD Mixed mix(uint32_t top, uint32_t rest)
 {
-    const uint64_t mask = key_mask(2 * m);
-    uint64_t x = (canonical * 0xd6e8feb86659fd93ull) & mask;
-    x ^= x >> m;
-    x = (x * 0xbf58476d1ce4e5b9ull) & mask;
-    x ^= x >> m;
-    return x;
+    uint32_t y = top * 0xd6e8feb9u + rest * 0x85ebca6bu;
+    y ^= y >> 15;
+    return Mixed{y * 0xbf58476du, rest};
 }
 
-// The key minimizers are chosen by: an odd 32-bit multiple of the line
-// hash's low 32 bits, with its low 3 bits cleared. Cheap on purpose: the scan
-// computes one per reference position, and it packs a window offset into the
-// 3 free bits so that one integer minimum per offset finds the leftmost (or,
-// on the other strand, the rightmost) smallest key. The line index comes
-// from the line hash's high bits; for every fixed line the multiples of its
-// low bits are spread evenly over the key range (a golden-ratio multiplier),
-// so picking small keys does not crowd lines.
-IBS_HD uint32_t rank_key_of(uint64_t lineHash) { return ((uint32_t)lineHash * 0x9e3779b1u) & ~7u; }
+IBS_HD Mixed mix_m(uint64_t canonical, uint32_t m)
+{
+    const uint32_t hb = 2 * m - 32;
+    return mix((uint32_t)(canonical >> hb), (uint32_t)canonical & ((1u << hb) - 1u));
+}
 
-IBS_HD uint32_t rank_key(uint64_t canonical, uint32_t m) { return rank_key_of(line_hash(canonical, m)); }
+// The line hash of a canonical m-mer: its hash as one 2m-bit number.
+IBS_HD uint64_t line_hash_of(const Mixed &x, uint32_t m) { return ((uint64_t)x.lo << (2 * m - 32)) | x.hi; }
+
+IBS_HD uint64_t line_hash(uint64_t canonical, uint32_t m) { return line_hash_of(mix_m(canonical, m), m); }
+
+// The key minimizers are chosen by: a multiple of the hash's words with its
+// low 5 bits clear, where the scan keeps a window offset and an orientation,
+// so that one integer minimum per step finds the leftmost smallest key. The
+// line index comes from lo's high bits; for every fixed line the multiples of
+// lo's low bits and of hi are spread evenly over the key range (golden-ratio
+// multipliers), so picking small keys does not crowd lines.
+IBS_HD uint32_t rank_key_of(const Mixed &x) { return x.lo * (0x9e3779b1u << 5) + x.hi * (0x94d049bbu << 5); }
+
+IBS_HD uint32_t rank_key(uint64_t canonical, uint32_t m) { return rank_key_of(mix_m(canonical, m)); }
 
 // The m-mer of C (2k-bit code, first base high) at offset o.
 IBS_HD uint64_t mmer_at(uint64_t C, uint32_t k, uint32_t o, uint32_t m)
@@ -96,39 +114,25 @@ IBS_HD uint64_t mmer_at(uint64_t C, uint32_t k, uint32_t o, uint32_t m)
     return (C >> (2 * (k - m - o))) & key_mask(2 * m);
 }
 
-// (o, s, C without the m-mer) part of the slot value: the minimizer's
-// offset o in C and its orientation s there (1 when it reads as the reverse
-// complement of its canonical form), then the k - m other bases: C rotated
-// left by 2o bits inside its 2k puts the m-mer on top and below it the bases
-// right of the m-mer followed by the o bases left of it. 2(k - m) + 4 <= 16
-// bits; m >= 16 and o <= k - m keep both shifts below 32.
-IBS_HD uint32_t slot_high(uint64_t C, uint32_t k, uint32_t o, uint32_t s)
+// (o, D without the m-mer) part of the slot value, D being the k-mer on the
+// strand where its minimizer reads as its canonical form and o the
+// minimizer's offset there: the k - m other bases are taken by rotating D
+// left by 2o bits inside its 2k, which puts the m-mer on top and below it the
+// bases right of the m-mer followed by the o bases left of it. 2(k - m) + 3
+// <= 17 bits; m >= 16 and o <= k - m keep both shifts below 32.
+IBS_HD uint32_t slot_high(uint64_t D, uint32_t k, uint32_t o)
 {
     const uint32_t m = m_of(k);
-    const uint32_t lo = (uint32_t)C, hi = (uint32_t)(C >> 32);
+    const uint32_t lo = (uint32_t)D, hi = (uint32_t)(D >> 32);
     const uint32_t rest = ((lo << (2 * o)) | (hi >> (2 * k - 32 - 2 * o))) & (uint32_t)key_mask(2 * (k - m));
-    return (((o << 1) | s) << (2 * (k - m))) | rest;
+    return (o << (2 * (k - m))) | rest;
 }
 
-// Minimizer offset of C by brute force (table build, single probes): the
-// leftmost m-mer with the smallest rank key.
-IBS_HD uint32_t minimizer_offset(uint64_t C, uint32_t k)
-{
-    const uint32_t m = m_of(k);
-    uint32_t best = 0xffffffffu, o = 0;
-    for (uint32_t j = 0; j < w_of(k); ++j) {
-        const uint32_t v = rank_key(canon_m(mmer_at(C, k, j, m), m), m);
-        if (j == 0 || v < best) {
-            best = v;
-            o = j;
-        }
-    }
-    return o;
-}
-
-// Sector of C inside its line: the top two bits of a golden-ratio multiple
-// of the code's two halves folded together.
-IBS_HD uint32_t sector_of(uint64_t C) { return (((uint32_t)C ^ (uint32_t)(C >> 32)) * 0x9e3779b1u) >> 30; }
+// Sector of a k-mer inside its line: the top two bits of a golden-ratio
+// multiple of its slot value's two halves folded together. The slot value
+// names the k-mer within its line, so it spreads the line's k-mers, and a
+// probe that has the slot value needs nothing else.
+IBS_HD uint32_t sector_of(uint32_t slotLo, uint32_t slotHi) { return ((slotLo ^ slotHi) * 0x9e3779b1u) >> 30; }
 
 // Line of a minimizer with line hash g (2m >= 32 bits) among nLines < 2^32:
 // the top 32 bits of g scaled to [0, nLines). Those of one line form an
@@ -145,37 +149,75 @@ IBS_HD uint64_t line_of(uint64_t g, uint32_t m, uint64_t nLines)
 #endif
 }
 
-// Bucket (32-byte sector index) and slot value of canonical k-mer C whose
-// minimizer sits at offset o with orientation s and line hash g.
-// hbits = 2m - floor(log2(nLines)).
-IBS_HD void place(uint64_t C, uint32_t k, uint32_t o, uint32_t s, uint64_t g, uint64_t nBuckets,
+// Bucket (32-byte sector index) and slot value of the k-mer D (either strand)
+// whose minimizer sits at offset o, with line hash g; s is 1 when D holds the
+// minimizer's reverse complement there: the k-mer then goes by its other
+// strand. hbits = 2m - floor(log2(nLines)).
+IBS_HD void place(uint64_t D, uint32_t k, uint32_t o, uint32_t s, uint64_t g, uint64_t nBuckets,
                   uint32_t hbits, uint64_t &bucket, uint64_t &slot)
 {
-    bucket = line_of(g, m_of(k), nBuckets / kSectorsPerLine) * kSectorsPerLine + sector_of(C);
-    slot = ((uint64_t)slot_high(C, k, o, s) << hbits) | (g & key_mask(hbits));
+    if (s) {
+        D = rc_m(D, k);
+        o = w_of(k) - 1 - o;
+    }
+    slot = ((uint64_t)slot_high(D, k, o) << hbits) | (g & key_mask(hbits));
+    bucket = line_of(g, m_of(k), nBuckets / kSectorsPerLine) * kSectorsPerLine +
+             sector_of((uint32_t)slot, (uint32_t)(slot >> 32));
 }
 
-// The same as place() where the slot value fits 32 bits (MZ8 sectors, joint
-// minimizer lines: hbits < 32 and the slot below 2^32 by their line counts),
-// in 32-bit arithmetic. Only bits 0 .. 2m-1 of g are read, so flag bits above
-// them do not matter.
-IBS_HD void place32(uint64_t C, uint32_t k, uint32_t o, uint32_t s, uint64_t g, uint64_t nBuckets,
-                    uint32_t hbits, uint64_t &bucket, uint64_t &slot)
+// The places of canonical k-mer C: where a scan that reads C looks (by C's
+// leftmost smallest rank key), and where one that reads the other strand
+// does. They are one place but for a k-mer whose smallest key occurs at
+// several offsets (a short tandem repeat: leftmost on one strand is rightmost
+// on the other), or whose minimizer is its own reverse complement; such a
+// k-mer is filed under both, so that a scan needs no look at which strand is
+// canonical. Returns how many (1 or 2; [0] is C's), and 0 for a code that is
+// not canonical: no scan asks for it, and a table keeps it in the stash, by
+// the code itself.
+IBS_HD uint32_t placements(uint64_t C, const TableGeom &g, uint64_t bucket[2], uint64_t slot[2])
 {
-    bucket = line_of(g, m_of(k), nBuckets / kSectorsPerLine) * kSectorsPerLine + sector_of(C);
-    const uint32_t low = (uint32_t)g & ((1u << hbits) - 1u);
-    slot = (slot_high(C, k, o, s) << hbits) | low;
+    const uint32_t k = g.k, m = m_of(k), w = w_of(k);
+    const uint64_t R = rc_m(C, k), mmask = key_mask(2 * m);
+    if (R < C)
+        return 0;
+    uint32_t best = 0, oL = 0, oR = 0;
+    uint64_t fL = 0, rL = 0, fR = 0, rR = 0;
+    Mixed xL{0, 0}, xR{0, 0};
+    for (uint32_t j = 0; j < w; ++j) {
+        // the m-mer at offset j and its reverse complement, from C's
+        const uint64_t f = (C >> (2 * (k - m - j))) & mmask, r = (R >> (2 * j)) & mmask;
+        const Mixed x = mix_m(f < r ? f : r, m);
+        const uint32_t key = rank_key_of(x);
+        if (j == 0 || key < best) {
+            best = key;
+            oL = j;
+            fL = f;
+            rL = r;
+            xL = x;
+        }
+        if (key <= best) {
+            oR = j;
+            fR = f;
+            rR = r;
+            xR = x;
+        }
+    }
+    place(C, k, oL, rL < fL, line_hash_of(xL, m), g.nBuckets, g.fpBits, bucket[0], slot[0]);
+    if (oL == oR && fL != rL)
+        return 1;
+    place(R, k, w - 1 - oR, fR < rR, line_hash_of(xR, m), g.nBuckets, g.fpBits, bucket[1], slot[1]);
+    return bucket[0] == bucket[1] && slot[0] == slot[1] ? 1 : 2;
 }
 
-// Slot value and bucket of a canonical k-mer (the build side, and single
-// probes): everything from C itself.
-IBS_HD void locate(uint64_t C, const TableGeom &g, uint64_t &bucket, uint64_t &slot)
+// The place where a probe for the k-mer's code looks; false for a code that is
+// not canonical.
+IBS_HD bool locate(uint64_t C, const TableGeom &g, uint64_t &bucket, uint64_t &slot)
 {
-    const uint32_t m = m_of(g.k);
-    const uint32_t o = minimizer_offset(C, g.k);
-    const uint64_t mm = mmer_at(C, g.k, o, m);
-    const uint64_t cm = canon_m(mm, m);
-    place(C, g.k, o, mm != cm ? 1u : 0u, line_hash(cm, m), g.nBuckets, g.fpBits, bucket, slot);
+    uint64_t b[2] = {0, 0}, s[2] = {0, 0};
+    const bool has = placements(C, g, b, s) != 0;
+    bucket = b[0];
+    slot = s[0];
+    return has;
 }
 
 } // namespace mz

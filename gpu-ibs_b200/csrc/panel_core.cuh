@@ -24,12 +24,12 @@
 // (at least 2^(2k-28) lines). Consecutive reference positions mostly share a
 // minimizer, so a warp's probes fall in few 128-byte lines instead of 32
 // random ones. A full sector keeps further keys in its partner sector (index
-// ^ 1, the same line; flag bit 25 of byte 31's word) and then in the stash
-// (bit 24).
+// ^ 1, the same line; flag bit 25 of byte 31's word), then in the line's
+// other two (bit 26) and then in the stash (bit 24).
 #pragma once
 
 #include "ibs_internal.cuh"
-#include "mz_core.cuh"
+#include "mz_scan.cuh"
 
 #include <vector>
 
@@ -41,6 +41,7 @@ constexpr uint32_t kSlots = 5;
 constexpr uint64_t kStashEmpty = ~0ull;
 constexpr uint32_t kStashFlag = 1u << 24;   // word 7: some key of this sector is in the stash
 constexpr uint32_t kPartnerFlag = 1u << 25; // word 7 (PM): some key of this sector is in its partner sector
+constexpr uint32_t kLineFlag = 1u << 26;    // word 7 (PM): ... or in one of the line's other two
 
 struct View {
     TableGeom g;
@@ -66,16 +67,14 @@ __device__ __forceinline__ uint32_t stash_mask(const View &t, uint64_t code)
 }
 
 // Sample mask of fingerprint (or slot value) fp in a sector's halves; 0
-// when no slot holds it.
+// when no slot holds it (a slot past the sector's count has an empty mask).
 __device__ __forceinline__ uint32_t sector_mask(const uint4 &v0, const uint4 &v1, uint32_t fp)
 {
-    const uint32_t cnt = (v1.w >> 16) & 0xff;
-    uint32_t m = 0;
-    m |= (0 < cnt && v0.x == fp) ? (v1.y & 0xffff) : 0u;
-    m |= (1 < cnt && v0.y == fp) ? (v1.y >> 16) : 0u;
-    m |= (2 < cnt && v0.z == fp) ? (v1.z & 0xffff) : 0u;
-    m |= (3 < cnt && v0.w == fp) ? (v1.z >> 16) : 0u;
-    m |= (4 < cnt && v1.x == fp) ? (v1.w & 0xffff) : 0u;
+    uint32_t m = v0.x == fp ? v1.y & 0xffffu : 0u;
+    m |= v0.y == fp ? v1.y >> 16 : 0u;
+    m |= v0.z == fp ? v1.z & 0xffffu : 0u;
+    m |= v0.w == fp ? v1.z >> 16 : 0u;
+    m |= v1.x == fp ? v1.w & 0xffffu : 0u;
     return m;
 }
 
@@ -89,55 +88,166 @@ __device__ __forceinline__ uint32_t bucket_mask(const uint4 &v0, const uint4 &v1
     return m;
 }
 
-// PM: the mask of the k-mer `code` with slot value `slot` whose home
-// sector r has halves v0, v1: the home sector, then (flagged) its partner
-// sector, then (flagged) the stash.
-__device__ __forceinline__ uint32_t pm_mask(const View &t, const uint4 &v0, const uint4 &v1, uint64_t r,
-                                            uint32_t slot, uint64_t code)
+// PM: the mask of a k-mer that its home sector r does not hold, from the
+// line's other sectors as the home sector's flags say (the stash is next).
+__device__ __forceinline__ uint32_t pm_line_mask(const View &t, uint32_t flags, uint64_t r, uint32_t slot)
 {
-    uint32_t m = sector_mask(v0, v1, slot);
-    if (m)
-        return m;
-    if (v1.w & kPartnerFlag) {
-        const uint4 w0 = __ldg(t.buckets + 2 * (r ^ 1)), w1 = __ldg(t.buckets + 2 * (r ^ 1) + 1);
-        m = sector_mask(w0, w1, slot);
-        if (m)
-            return m;
+    uint32_t m = 0;
+    auto look = [&](uint64_t x) { return sector_mask(__ldg(t.buckets + 2 * x), __ldg(t.buckets + 2 * x + 1), slot); };
+    if (flags & kPartnerFlag) {
+        m = look(r ^ 1);
+        if (!m && (flags & kLineFlag))
+            m = look(r ^ 2) | look(r ^ 3);
     }
-    return (v1.w & kStashFlag) ? stash_mask(t, code) : 0u;
+    return m;
 }
 
-// Home sector and stored fingerprint (P5x48) or slot value (PM) of a key.
-__device__ __forceinline__ void joint_place(const View &t, uint64_t code, uint64_t &r, uint32_t &fp)
+// Home sectors and stored fingerprints (P5x48) or slot values (PM) of a key;
+// returns how many places it has (mz::placements; none: the stash only).
+__device__ __forceinline__ uint32_t joint_places(const View &t, uint64_t code, uint64_t r[2], uint32_t fp[2])
 {
     if (t.g.format == FMT_PANEL_MZ) {
-        uint64_t slot;
-        mz::locate(code, t.g, r, slot);
-        fp = (uint32_t)slot;
-        return;
+        uint64_t slot[2];
+        const uint32_t n = mz::placements(code, t.g, r, slot);
+        fp[0] = n ? (uint32_t)slot[0] : 0u;
+        fp[1] = n == 2 ? (uint32_t)slot[1] : 0u;
+        return n;
     }
     const uint64_t h = perm_hash(code, t.g.bits);
-    r = bucket_of(h, t.g);
-    fp = (uint32_t)fp_of(h, t.g);
+    r[0] = bucket_of(h, t.g);
+    fp[0] = (uint32_t)fp_of(h, t.g);
+    return 1;
 }
 
 __device__ __forceinline__ uint32_t lookup_mask(const View &t, uint64_t code)
 {
+    uint64_t r[2];
+    uint32_t fp[2];
+    if (!joint_places(t, code, r, fp))
+        return stash_mask(t, code);
+    uint4 v0, v1;
+    load_sector(t.buckets + 2 * r[0], v0, v1);
     if (t.g.format == FMT_PANEL_MZ) {
-        uint64_t r;
-        uint32_t slot;
-        joint_place(t, code, r, slot);
-        const uint4 v0 = __ldg(t.buckets + 2 * r), v1 = __ldg(t.buckets + 2 * r + 1);
-        return pm_mask(t, v0, v1, r, slot, code);
+        uint32_t m = sector_mask(v0, v1, fp[0]);
+        if (!m)
+            m = pm_line_mask(t, v1.w, r[0], fp[0]);
+        return !m && (v1.w & kStashFlag) ? stash_mask(t, code) : m;
     }
-    const uint64_t h = perm_hash(code, t.g.bits);
-    const uint64_t r = bucket_of(h, t.g);
-    const uint4 v0 = __ldg(t.buckets + 2 * r), v1 = __ldg(t.buckets + 2 * r + 1);
-    uint32_t m = bucket_mask(v0, v1, (uint32_t)fp_of(h, t.g));
-    if (m & 0x80000000u)
-        m = stash_mask(t, code);
-    return m;
+    const uint32_t m = bucket_mask(v0, v1, fp[0]);
+    return m & 0x80000000u ? stash_mask(t, code) : m;
 }
+
+// The same of the k-mer at packed base G, out of line (see dev::mz_elsewhere);
+// flags is the home sector's flag byte.
+static __device__ __noinline__ uint32_t elsewhere_mask(const View *t, const uint64_t *__restrict__ seq,
+                                                       const uint64_t *__restrict__ mask, uint64_t G, uint32_t k,
+                                                       uint32_t line, uint32_t slot, uint32_t flags)
+{
+    const uint32_t m =
+        pm_line_mask(*t, flags << 24, (uint64_t)line * mz::kSectorsPerLine + mz::sector_of(slot, 0), slot);
+    if (m || !((flags << 24) & kStashFlag))
+        return m;
+    bool acgt;
+    return stash_mask(*t, dev::canonical_at(seq, mask, G, k, key_mask(2 * k), key_mask(k), acgt));
+}
+
+// The sample masks of a block's positions (MzWarp::block has located it): m[i]
+// is position 32 i + lane's, valid[i] whether it has a k-mer. RANGE: sectors
+// outside [bLo, bHi) count as empty (they read sector bLo).
+template <uint32_t K, bool RANGE>
+__device__ __forceinline__ void mz_masks(const dev::MzShared<FMT_B8X32> *sh, const View &t,
+                                         const uint64_t *__restrict__ seq, const uint64_t *__restrict__ mask,
+                                         uint64_t blockBase, uint32_t lane, uint64_t bLo, uint64_t bHi,
+                                         uint32_t (&m)[4], bool (&valid)[4])
+{
+    uint32_t more = 0; // 3 bits a position: the flags of a full sector that does not hold it
+    {
+        dev::MzSectors s;
+        bool mine[4];
+        if (RANGE) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                s.record(sh, i, 32 * i + lane);
+                const uint64_t r = s.sector(i);
+                mine[i] = s.valid(i) && r >= bLo && r < bHi;
+                load_sector(t.buckets + 2 * (mine[i] ? r : bLo), s.v0[i], s.v1[i]);
+            }
+        } else {
+            s.load(sh, t.buckets, lane);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            valid[i] = s.valid(i);
+            if (!RANGE)
+                mine[i] = valid[i];
+            m[i] = mine[i] ? sector_mask(s.v0[i], s.v1[i], s.slot[i]) : 0u;
+            if (mine[i] && !m[i])
+                more |= ((s.v1[i].w >> 24) & 7u) << (3 * i);
+        }
+    }
+    while (more) {
+        const int i = (__ffs(more) - 1) / 3;
+        dev::MzSectors s;
+        s.record(sh, 0, 32 * i + lane);
+        const uint32_t x = elsewhere_mask(&t, seq, mask, blockBase + 32 * i + lane, K, s.line[0], s.slot[0],
+                                          (more >> (3 * i)) & 7u);
+        m[0] = i == 0 ? x : m[0];
+        m[1] = i == 1 ? x : m[1];
+        m[2] = i == 2 ? x : m[2];
+        m[3] = i == 3 ? x : m[3];
+        more &= ~(7u << (3 * i));
+    }
+}
+
+// Statistics of up to 16 samples over a span's blocks of 128 positions, from
+// the last block to the first. A block's four 16-bit masks a lane are two
+// 32 x 32 bit matrices (positions by samples), transposed by five shuffles
+// each: lane j then has sample j's hits of the block's first 64 positions and
+// lane 16 + j those of its last 64, so that all 32 lanes summarise
+// (16 ballots and a select each gave the words to 16 lanes only).
+struct JointFold {
+    Seg32 acc{0, 0, 0, 0, 0, 0}; // lane j < 16: sample j, the blocks so far
+    uint32_t amount[5], keep[5];
+
+    __device__ __forceinline__ explicit JointFold(uint32_t lane)
+    {
+        const uint32_t M[5] = {0x0000ffffu, 0x00ff00ffu, 0x0f0f0f0fu, 0x33333333u, 0x55555555u};
+#pragma unroll
+        for (int i = 0; i < 5; ++i) {
+            const uint32_t s = 16u >> i;
+            amount[i] = lane & s ? 32 - s : s;
+            keep[i] = lane & s ? ~M[i] : M[i];
+        }
+    }
+
+    // Bit i of lane l's result is bit l of lane i's x.
+    __device__ __forceinline__ uint32_t transpose(uint32_t x) const
+    {
+#pragma unroll
+        for (int i = 0; i < 5; ++i) {
+            const uint32_t y = __shfl_xor_sync(dev::FULL_MASK, x, 16 >> i);
+            x = (x & keep[i]) | (__funnelshift_l(y, y, amount[i]) & ~keep[i]);
+        }
+        return x;
+    }
+
+    // m: the lane's masks of positions 32 i + lane; valid: whether they count.
+    __device__ __forceinline__ void push(const uint32_t (&m)[4], const bool (&valid)[4], uint32_t lane, int k)
+    {
+        const uint32_t V0 = __ballot_sync(dev::FULL_MASK, valid[0]), V1 = __ballot_sync(dev::FULL_MASK, valid[1]),
+                       V2 = __ballot_sync(dev::FULL_MASK, valid[2]), V3 = __ballot_sync(dev::FULL_MASK, valid[3]);
+        const uint32_t Ha = transpose(m[0] | m[2] << 16), Hb = transpose(m[1] | m[3] << 16);
+        Seg32 s = seg32_combine(block_seg32(lane < 16 ? V0 : V2, Ha, k), block_seg32(lane < 16 ? V1 : V3, Hb, k), k);
+        Seg32 o;
+        o.total = __shfl_down_sync(dev::FULL_MASK, s.total, 16);
+        o.obs = __shfl_down_sync(dev::FULL_MASK, s.obs, 16);
+        o.lead = __shfl_down_sync(dev::FULL_MASK, s.lead, 16);
+        o.trail = __shfl_down_sync(dev::FULL_MASK, s.trail, 16);
+        o.gaps = __shfl_down_sync(dev::FULL_MASK, s.gaps, 16);
+        o.dist = __shfl_down_sync(dev::FULL_MASK, s.dist, 16);
+        acc = seg32_combine(seg32_combine(s, o, k), acc, k);
+    }
+};
 
 // Block statistics of one sample from its valid (V) and hit (H) masks,
 // computed by one lane with bit operations: the gaps between hits are the

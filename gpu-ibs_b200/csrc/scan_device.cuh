@@ -15,15 +15,16 @@ constexpr uint32_t FULL_MASK = 0xffffffffu;
 // every 32 blocks (and at the end of the span) each lane summarises its own
 // block with 32-bit operations and a shuffle tree combines the 32 summaries
 // in block order into the running summary. A block costs the keeping lane a
-// compare and two selects.
-struct LaneFold {
+// compare and two selects. REVERSED: the blocks come from the span's last to
+// its first, and fill the lanes from 31 down.
+template <bool REVERSED = false> struct LaneFold {
     uint32_t v = 0, h = 0; // this lane's block since the last flush
     uint32_t n = 0;        // blocks since the last flush (warp-uniform)
     Seg32 acc{0, 0, 0, 0, 0, 0};
 
     __device__ __forceinline__ void push(uint32_t V, uint32_t H, uint32_t lane, int k)
     {
-        if (lane == n) {
+        if (lane == (REVERSED ? 31u - n : n)) {
             v = V;
             h = H;
         }
@@ -33,7 +34,7 @@ struct LaneFold {
 
     __device__ __forceinline__ void flush(int k)
     {
-        Seg32 s = block_seg32(v, h, k); // lanes past n hold empty blocks
+        Seg32 s = block_seg32(v, h, k); // lanes without a block hold an empty one
 #pragma unroll
         for (uint32_t off = 1; off < 32; off <<= 1) {
             Seg32 o;
@@ -45,7 +46,7 @@ struct LaneFold {
             o.dist = __shfl_down_sync(FULL_MASK, s.dist, off);
             s = seg32_combine(s, o, k); // right for lanes that are multiples of 2 off
         }
-        acc = seg32_combine(acc, s, k); // lane 0's is the span so far
+        acc = REVERSED ? seg32_combine(s, acc, k) : seg32_combine(acc, s, k); // lane 0's is the span so far
         v = h = n = 0;
     }
 

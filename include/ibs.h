@@ -263,7 +263,7 @@ ibs_status ibs_scan_panel(ibs_table *const *tables, uint32_t n_tables, ibs_refer
  * (opts->force_format): 3 = hash sectors (P5x48: five fingerprints and
  * sample masks per 32-byte sector, any k); 7 = the same sectors on minimizer
  * lines (16 <= k <= 27, at least 2^(2k-28) lines; consecutive positions
- * share 128-byte lines, a full sector spills into its partner sector, then
+ * share 128-byte lines, a full sector spills into the line's others, then
  * the stash; default load 1.5 keys per sector); 0 = 7 where it applies and its
  * minimum size does not oversize the table, else 3. opts->keys_per_bucket: keys
  * per sector (0 = the tuned panel_keys_per_bucket for 3, 1.5 for 7). Samples are added one at a
@@ -431,8 +431,10 @@ ibs_status ibs_scan_noalloc(ibs_table *t, const uint64_t *seq2bit_dev, const uin
  * fields keep the current value. */
 typedef struct ibs_tuning {
     uint32_t span_len;         /* k-mer positions per warp task (multiple of 128) */
-    uint32_t blocks_in_flight; /* 32-position blocks each lane keeps in flight: 1, 2, 4 or 8 */
-    uint32_t block_threads;    /* threads per CTA: 128, 256 or 512 */
+    uint32_t blocks_in_flight; /* 32-position blocks each lane keeps in flight: 1, 2, 4 or 8 (hash buckets;
+                                  the minimizer-line scan always has 4) */
+    uint32_t block_threads;    /* threads per CTA: 128, 256 or 512 (hash buckets; the minimizer-line scan's
+                                  CTAs have 256) */
     uint32_t ctas_per_sm;      /* resident CTAs per SM the grid is sized for */
     double keys_per_bucket;    /* default load of new tables */
     uint32_t table_format;     /* default format of new tables (0 = automatic, 4 = minimizer buckets) */
