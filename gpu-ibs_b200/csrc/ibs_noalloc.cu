@@ -13,6 +13,7 @@
 // The kernels are the scan of ibs_scan.cu with its per-window plan replaced
 // by per-contig window arithmetic, so nothing per window has to be uploaded.
 #include "ibs_internal.cuh"
+#include "mz_scan.cuh"
 #include "scan_device.cuh"
 
 #include <cub/block/block_scan.cuh>
@@ -126,6 +127,45 @@ __device__ __forceinline__ uint32_t last_le(const ContigDesc *cd, uint32_t n, ui
     return lo;
 }
 
+// Span s's positions [p0, p1) of a window of nPos positions whose first base
+// is packed base `base`.
+struct SpanAt {
+    uint64_t base, nPos;
+    uint32_t p0, p1;
+};
+
+__device__ __forceinline__ SpanAt span_at(const ContigDesc *__restrict__ cd, uint32_t n, uint32_t W, uint32_t k,
+                                          uint64_t s)
+{
+    const uint32_t c = last_le(cd, n, s, true);
+    const uint64_t L = cd[c].len;
+    const ContigWin cw = contig_windows(L, W, k);
+    uint64_t sc = s - cd[c].span0, i, nPos;
+    if (sc < cw.nFull * cw.spw) {
+        i = sc / cw.spw;
+        sc -= i * cw.spw;
+        nPos = (uint64_t)W - k + 1;
+    } else {
+        sc -= cw.nFull * cw.spw;
+        i = cw.nFull;
+        for (;;) {
+            nPos = window_npos(L, i, W, k);
+            const uint64_t sp = spans_of(nPos);
+            if (sc < sp)
+                break;
+            sc -= sp;
+            ++i;
+        }
+    }
+    SpanAt a;
+    a.base = cd[c].base + i * ((uint64_t)W - k);
+    a.nPos = nPos;
+    a.p0 = (uint32_t)sc * kSpanLen;
+    a.p1 = (uint32_t)(a.p0 + kSpanLen < nPos ? a.p0 + kSpanLen : nPos);
+    return a;
+}
+
+// Hash-bucket tables.
 template <uint32_t FMT, int NB>
 __global__ void __launch_bounds__(256) k_na_spans(TableView t, const uint64_t *__restrict__ seq,
                                                   const uint64_t *__restrict__ mask,
@@ -140,64 +180,34 @@ __global__ void __launch_bounds__(256) k_na_spans(TableView t, const uint64_t *_
     const uint64_t kmask = key_mask(2 * k);
     const uint64_t kbits = (1ull << k) - 1;
     for (uint64_t s = warp; s < nSpans; s += nWarps) {
-        const uint32_t c = last_le(cd, n, s, true);
-        const uint64_t L = cd[c].len;
-        const ContigWin cw = contig_windows(L, W, k);
-        uint64_t sc = s - cd[c].span0, i, nPos;
-        if (sc < cw.nFull * cw.spw) {
-            i = sc / cw.spw;
-            sc -= i * cw.spw;
-            nPos = (uint64_t)W - k + 1;
-        } else {
-            sc -= cw.nFull * cw.spw;
-            i = cw.nFull;
-            for (;;) {
-                nPos = window_npos(L, i, W, k);
-                const uint64_t sp = spans_of(nPos);
-                if (sc < sp)
-                    break;
-                sc -= sp;
-                ++i;
-            }
-        }
-        const uint64_t base = cd[c].base + i * ((uint64_t)W - k);
-        const uint32_t p0 = (uint32_t)sc * kSpanLen;
-        const uint32_t p1 = (uint32_t)(p0 + kSpanLen < nPos ? p0 + kSpanLen : nPos);
+        const SpanAt sp = span_at(cd, n, W, k, s);
         dev::LaneFold<> fold;
-        for (uint32_t p = p0; p < p1; p += 32 * NB) {
+        for (uint32_t p = sp.p0; p < sp.p1; p += 32 * NB) {
             uint4 v0[NB], v1[NB];
             uint64_t code[NB], fp[NB];
             bool valid[NB];
 #pragma unroll
             for (int b = 0; b < NB; ++b) {
                 const uint32_t q = p + 32 * b + lane;
-                const bool inSpan = q < p1;
-                const uint64_t G = base + (inSpan ? q : p0);
+                const bool inSpan = q < sp.p1;
+                const uint64_t G = sp.base + (inSpan ? q : sp.p0);
                 bool acgt;
                 code[b] = dev::canonical_at(seq, mask, G, k, kmask, kbits, acgt);
                 valid[b] = inSpan && acgt;
                 const uint64_t h = perm_hash(code[b], t.g.bits);
                 const uint64_t r = bucket_of(h, t.g);
                 fp[b] = fp_of(h, t.g);
-                if (valid[b] && !is_mz(FMT)) {
-                    v0[b] = __ldg(t.buckets + 2 * r);
-                    v1[b] = __ldg(t.buckets + 2 * r + 1);
-                } else {
-                    v0[b] = make_uint4(0, 0, 0, 0);
-                    v1[b] = make_uint4(0, 0, 0, 0);
-                }
+                v0[b] = make_uint4(0, 0, 0, 0);
+                v1[b] = make_uint4(0, 0, 0, 0);
+                if (valid[b])
+                    load_sector(t.buckets + 2 * r, v0[b], v1[b]);
             }
 #pragma unroll
             for (int b = 0; b < NB; ++b) {
                 bool hit = false;
                 if (valid[b]) {
-                    if constexpr (FMT == FMT_MZ8 || FMT == FMT_MZ6) {
-                        // minimizer table: each lane finds its k-mer's minimizer on its own
-                        hit = table_lookup<FMT>(t, code[b]);
-                    } else {
-                        const uint32_t m = bucket_match<FMT>(v0[b], v1[b], fp[b]);
-                        hit = m == 1u || (m == 2u && stash_lookup(t, code[b]));
-                    }
+                    const uint32_t m = bucket_match<FMT>(v0[b], v1[b], fp[b]);
+                    hit = m == 1u || (m == 2u && stash_lookup(t, code[b]));
                 }
                 const uint32_t V = __ballot_sync(dev::FULL_MASK, valid[b]);
                 const uint32_t H = __ballot_sync(dev::FULL_MASK, hit);
@@ -205,6 +215,29 @@ __global__ void __launch_bounds__(256) k_na_spans(TableView t, const uint64_t *_
             }
         }
         const SegStats acc = fold.finish((int)k);
+        if (lane == 0)
+            out[s] = acc;
+    }
+}
+
+// Minimizer-line tables: the window scan's located blocks (mz_scan.cuh). A
+// lane that looks for its k-mer's minimizer alone hashes w m-mers a position:
+// 250 Mbp at k = 25 took 6.8 ms so, 1.7 ms this way.
+template <uint32_t K, uint32_t SEC>
+__global__ void __launch_bounds__(256, 3) k_na_spans_mz(const __grid_constant__ TableView t,
+                                                        const uint64_t *__restrict__ seq,
+                                                        const uint64_t *__restrict__ mask,
+                                                        const ContigDesc *__restrict__ cd, uint32_t n, uint32_t W,
+                                                        uint64_t nSpans, SegStats *__restrict__ out)
+{
+    __shared__ dev::MzShared<SEC> shared[8];
+    const uint32_t lane = dev::lane_id();
+    const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+    const uint64_t nWarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    for (uint64_t s = warp; s < nSpans; s += nWarps) {
+        const SpanAt sp = span_at(cd, n, W, K, s);
+        const SegStats acc = dev::mz_span_stats<K, SEC>(&shared[threadIdx.x >> 5], t, seq, mask, sp.base + sp.p0,
+                                                        sp.p1 - sp.p0, sp.base + sp.nPos - 1 + (K - 1), lane);
         if (lane == 0)
             out[s] = acc;
     }
@@ -351,12 +384,11 @@ extern "C" ibs_status ibs_scan_noalloc(ibs_table *t, const uint64_t *seq2bit_dev
         if (t->geom.format == FMT_B8X32)
             k_na_spans<FMT_B8X32, kNB><<<grid, 256, 0, st>>>(t->view(), seq2bit_dev, nmask_dev, dDesc,
                                                              n_contigs, W, nSpans, dSpans);
-        else if (t->geom.format == FMT_MZ8)
-            k_na_spans<FMT_MZ8, kNB><<<grid, 256, 0, st>>>(t->view(), seq2bit_dev, nmask_dev, dDesc,
-                                                           n_contigs, W, nSpans, dSpans);
-        else if (t->geom.format == FMT_MZ6)
-            k_na_spans<FMT_MZ6, kNB><<<grid, 256, 0, st>>>(t->view(), seq2bit_dev, nmask_dev, dDesc,
-                                                           n_contigs, W, nSpans, dSpans);
+        else if (is_mz(t->geom.format))
+            with_mz_table(t->geom, [&](auto K, auto SEC) {
+                k_na_spans_mz<K.value, SEC.value><<<grid, 256, 0, st>>>(t->view(), seq2bit_dev, nmask_dev, dDesc,
+                                                                        n_contigs, W, nSpans, dSpans);
+            });
         else
             k_na_spans<FMT_B6X40, kNB><<<grid, 256, 0, st>>>(t->view(), seq2bit_dev, nmask_dev, dDesc,
                                                              n_contigs, W, nSpans, dSpans);

@@ -430,15 +430,6 @@ int grid_for(uint64_t n)
     return (int)std::max<uint64_t>(1, std::min<uint64_t>((n + 255) / 256, (uint64_t)sm_count() * 16));
 }
 
-// Calls f with a minimizer-line joint table's k as a compile-time constant.
-template <uint32_t K = 16, typename F> void with_pm_k(uint32_t k, F &&f)
-{
-    if (k == K)
-        f(std::integral_constant<uint32_t, K>{});
-    else if constexpr (K < 27)
-        with_pm_k<K + 1>(k, f);
-}
-
 // Expected fraction of keys beyond a bucket's kSlots slots when the keys per
 // bucket are Poisson(lam).
 double overflow_fraction(double lam)
@@ -806,7 +797,7 @@ static ibs_status enqueue_spans(ibs_panel_table *p, const ibs_reference *ref, ui
     if (passes <= 1) {
         if (p->geom.format != FMT_PANEL_MZ)
             return go(k_panel_spans<NB, kScan>, 0, 0, false);
-        with_pm_k(p->geom.k, [&](auto K) { s = go(k_panel_spans_mz<K.value, kScan>, 0, 0, false); });
+        with_mz_k<16, 27>(p->geom.k, [&](auto K) { s = go(k_panel_spans_mz<K.value, kScan>, 0, 0, false); });
         return s;
     }
     for (uint32_t i = 0; i < passes && s == IBS_OK; ++i) {
@@ -814,7 +805,7 @@ static ibs_status enqueue_spans(ibs_panel_table *p, const ibs_reference *ref, ui
         if (p->geom.format != FMT_PANEL_MZ)
             s = go(k_panel_spans<NB, kMaskPass>, bLo, bHi, i == 0);
         else
-            with_pm_k(p->geom.k, [&](auto K) { s = go(k_panel_spans_mz<K.value, kMaskPass>, bLo, bHi, i == 0); });
+            with_mz_k<16, 27>(p->geom.k, [&](auto K) { s = go(k_panel_spans_mz<K.value, kMaskPass>, bLo, bHi, i == 0); });
     }
     return s == IBS_OK ? go(k_panel_spans<NB, kStats>, 0, 0, false) : s;
 }

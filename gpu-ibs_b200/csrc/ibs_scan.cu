@@ -286,22 +286,17 @@ void plan_windows(ScanPlan &p, const std::vector<uint64_t> &lens,
 }
 
 // Minimizer-line tables: one kernel for every k that the format takes.
-template <uint32_t K, uint32_t SEC>
 static void launch_mz(const ibs_table *t, const uint64_t *dSeq, const uint64_t *dMask, const ScanPlan &p, uint64_t s0,
                       uint64_t s1, SegStats *dSpans, cudaStream_t st)
 {
-    if constexpr (SEC == FMT_B8X32 ? K >= 16 && K <= 27 : K >= 16 && K <= 31) {
-        if (t->geom.k != K) {
-            launch_mz<K + 1, SEC>(t, dSeq, dMask, p, s0, s1, dSpans, st);
-            return;
-        }
-        const uint64_t warpsPerCta = kMzThreads / 32;
-        const uint64_t want = (s1 - s0 + warpsPerCta - 1) / warpsPerCta;
-        const uint64_t cap = (uint64_t)sm_count() * tuning().ctas_per_sm * 2; // ctas_per_sm counts CTAs of 512
-        const int grid = (int)std::max<uint64_t>(1, std::min(want, cap));
-        k_scan_spans_mz<K, SEC><<<grid, kMzThreads, 0, st>>>(t->view(), dSeq, dMask, p.dWin, p.dSpan0, (uint32_t)p.nWin,
-                                                            s0, s1, p.spanLen, dSpans);
-    }
+    const uint64_t warpsPerCta = kMzThreads / 32;
+    const uint64_t want = (s1 - s0 + warpsPerCta - 1) / warpsPerCta;
+    const uint64_t cap = (uint64_t)sm_count() * tuning().ctas_per_sm * 2; // ctas_per_sm counts CTAs of 512
+    const int grid = (int)std::max<uint64_t>(1, std::min(want, cap));
+    with_mz_table(t->geom, [&](auto K, auto SEC) {
+        k_scan_spans_mz<K.value, SEC.value><<<grid, kMzThreads, 0, st>>>(
+            t->view(), dSeq, dMask, p.dWin, p.dSpan0, (uint32_t)p.nWin, s0, s1, p.spanLen, dSpans);
+    });
 }
 
 template <uint32_t FMT>
@@ -353,10 +348,8 @@ static ibs_status launch_spans(const ibs_table *t, const uint64_t *dSeq, const u
         launch_spans_wide(t, dSeq, dMask, p, s0, s1, dSpans, st);
     else if (t->geom.format == FMT_B8X32)
         launch_spans_fmt<FMT_B8X32>(t, dSeq, dMask, p, s0, s1, dSpans, st);
-    else if (t->geom.format == FMT_MZ8)
-        launch_mz<16, FMT_B8X32>(t, dSeq, dMask, p, s0, s1, dSpans, st);
-    else if (t->geom.format == FMT_MZ6)
-        launch_mz<16, FMT_B6X40>(t, dSeq, dMask, p, s0, s1, dSpans, st);
+    else if (is_mz(t->geom.format))
+        launch_mz(t, dSeq, dMask, p, s0, s1, dSpans, st);
     else
         launch_spans_fmt<FMT_B6X40>(t, dSeq, dMask, p, s0, s1, dSpans, st);
     IBS_LAUNCHED();

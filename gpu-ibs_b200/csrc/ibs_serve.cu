@@ -687,14 +687,12 @@ __global__ void __launch_bounds__(256, 3) k_serve_persistent(const Ctrl *ctrl, S
 
 // Calls f with the server's k as a compile-time constant: every k that a
 // minimizer table can have, else 0.
-template <uint32_t K = 16, typename F> void with_k(uint32_t k, F &&f)
+template <typename F> void with_k(uint32_t k, F &&f)
 {
-    if (k < 16 || K > 31)
+    if (k < 16 || k > 31)
         f(std::integral_constant<uint32_t, 0>{});
-    else if (k == K)
-        f(std::integral_constant<uint32_t, K <= 31 ? K : 0>{});
-    else if constexpr (K <= 31)
-        with_k<K + 1>(k, f);
+    else
+        with_mz_k<16, 31>(k, f);
 }
 
 // First-fit allocator of [offset, offset+size) ranges of a pool.

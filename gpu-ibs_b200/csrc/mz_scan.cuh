@@ -6,6 +6,8 @@
 #include "ibs_internal.cuh"
 #include "scan_device.cuh"
 
+#include <type_traits>
+
 namespace ibs {
 namespace dev {
 
@@ -415,4 +417,23 @@ __device__ __forceinline__ SegStats mz_span_stats(MzShared<SEC> *sh, const Table
 }
 
 } // namespace dev
+
+// Calls f with a minimizer table's k (16 <= k <= last) as a compile-time
+// constant.
+template <uint32_t K, uint32_t LAST, typename F> void with_mz_k(uint32_t k, F &&f)
+{
+    if (k == K)
+        f(std::integral_constant<uint32_t, K>{});
+    else if constexpr (K < LAST)
+        with_mz_k<K + 1, LAST>(k, f);
+}
+
+// The same with the sector layout of a table's format: f(K, SEC).
+template <typename F> void with_mz_table(const TableGeom &g, F &&f)
+{
+    if (g.format == FMT_MZ8)
+        with_mz_k<16, 27>(g.k, [&](auto K) { f(K, std::integral_constant<uint32_t, FMT_B8X32>{}); });
+    else
+        with_mz_k<16, 31>(g.k, [&](auto K) { f(K, std::integral_constant<uint32_t, FMT_B6X40>{}); });
+}
 } // namespace ibs

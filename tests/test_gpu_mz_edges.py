@@ -80,3 +80,37 @@ def test_full_lines(fmt, kpb):
     assert odd.probe(q).all()
     ref = ib.Reference(*ib.pack_ascii(seqs))
     assert np.array_equal(ib.scan(t, ref, 500), ib.scan(h, ref, 500))
+
+
+@pytest.mark.parametrize("k", range(16, 32))
+def test_coverage_edges(k):
+    seqs, codes = _world(k)
+    rng = np.random.default_rng(k)
+    for n in (4063, 4064, 4065, 4064 + k, 8128 + k - 1):  # around the mapper's spans
+        seqs.append(np.frombuffer(b"ACGT", np.uint8)[rng.integers(0, 4, n)].tobytes())
+        codes = np.concatenate([codes, orc.canonical_codes(seqs[-1], k)[::3]])
+    codes = np.unique(codes)
+    ref = ib.Reference(*ib.pack_ascii(seqs))
+    want = ib.map_coverage(ib.Table.from_codes(codes, len(codes), k, on_device=False, force_format=5), ref)
+    assert want.max() > 1
+    for fmt in (4, 6) if k <= 27 else (6,):
+        t = ib.Table.from_codes(codes, len(codes), k, on_device=False, force_format=fmt)
+        assert np.array_equal(ib.map_coverage(t, ref), want), (k, fmt)
+
+
+@pytest.mark.parametrize("k", [16, 21, 25, 27, 28, 31])
+def test_noalloc_edges(k):
+    import torch
+    seqs, codes = _world(k)
+    seq, mask, lens = ib.pack_ascii(seqs)
+    ref = ib.Reference(seq, mask, lens)
+    dseq, dmask = torch.from_numpy(seq.view(np.int64)).cuda(), torch.from_numpy(mask.view(np.int64)).cuda()
+    h = ib.Table.from_codes(codes, len(codes), k, on_device=False, force_format=5)
+    for fmt in (4, 6) if k <= 27 else (6,):
+        t = ib.Table.from_codes(codes, len(codes), k, on_device=False, force_format=fmt)
+        for W in (k + 1, k + 128, 1000, 20_000):
+            want = ib.scan(h, ref, W)
+            rows = torch.zeros((len(want), 6), dtype=torch.int32, device="cuda")
+            ib.scan_noalloc(t, dseq, dmask, lens, W, rows, len(want), torch.cuda.current_stream().cuda_stream)
+            torch.cuda.synchronize()
+            assert np.array_equal(rows.cpu().numpy(), want.view(np.int32).reshape(-1, 6)), (k, fmt, W)
