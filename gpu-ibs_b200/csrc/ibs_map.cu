@@ -12,6 +12,7 @@
 // device: each 8192-value tile is sized, the tile offsets are summed on the
 // host, and a second pass ranks each thread's characters with a block scan.
 #include "ibs_internal.cuh"
+#include "mz_scan.cuh"
 #include "scan_device.cuh"
 
 #include <cub/block/block_scan.cuh>
@@ -24,7 +25,7 @@
 namespace ibs {
 namespace map {
 
-constexpr uint32_t kSpan = 4096;       // bases per warp task
+constexpr uint32_t kSpan = 4064;       // bases per warp task: with the 32 starts before it, 32 blocks of 128
 constexpr uint32_t kThreads = 256;
 constexpr uint32_t kPerThread = 32;
 constexpr uint32_t kTile = kThreads * kPerThread; // coverage values per text tile
@@ -76,6 +77,57 @@ __global__ void __launch_bounds__(256) k_map_spans(TableView t, const uint64_t *
             if (p + lane < sp.b)
                 cov[sp.out + p + lane] = (uint8_t)__popcll((M >> (33 + lane - k)) & kbits);
             prev = H;
+        }
+    }
+}
+
+// Minimizer-line tables: the hits of the span's starts and of the 32 before it
+// from the window scan's located blocks (mz_scan.cuh), which run from the
+// last to the first, so a 32-base piece is counted when the hits of the
+// starts before it are known. (A lane that looks for its k-mer's minimizer
+// alone hashes w m-mers a position: 64 Mbp at k = 25 took 1.74 ms so.)
+template <uint32_t K, uint32_t SEC>
+__global__ void __launch_bounds__(256, 3) k_map_spans_mz(const __grid_constant__ TableView t,
+                                                         const uint64_t *__restrict__ seq,
+                                                         const uint64_t *__restrict__ mask,
+                                                         const Span *__restrict__ spans, uint64_t nSpans,
+                                                         uint8_t *__restrict__ cov)
+{
+    __shared__ dev::MzShared<SEC> shared[8];
+    dev::MzShared<SEC> *sh = &shared[threadIdx.x >> 5];
+    const uint32_t lane = dev::lane_id();
+    const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+    const uint64_t nWarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    for (uint64_t i = warp; i < nSpans; i += nWarps) {
+        const Span sp = spans[i];
+        const uint32_t first = sp.a >= 32 ? sp.a - 32 : 0; // the first start looked at
+        const uint32_t last = min(sp.b, sp.nPos);           // past the last one
+        uint32_t later = 0; // hits of the 32 starts from p on
+        // bases p .. p + 31, given the hits of the 32 starts before p
+        auto count = [&](uint32_t p, uint32_t prev) {
+            const uint64_t M = ((uint64_t)later << 32) | prev;
+            const uint32_t q = p + lane;
+            if (q >= sp.a && q < sp.b)
+                cov[sp.out + q] = (uint8_t)__popcll((M >> (33 + lane - K)) & ((1ull << K) - 1));
+        };
+        uint32_t p = first;
+        if (last > first) {
+            const uint64_t base = sp.base + first;
+            dev::MzWarp<K, SEC> blocks(sh, t.g, seq, mask, base, last - first, sp.base + sp.nPos - 1 + (K - 1), lane);
+            blocks.start();
+            p = first + dev::kMzBlock * blocks.blocks(); // at most K - 1 of the span's bases lie past it
+            for (int b = blocks.blocks() - 1; b >= 0; --b) {
+                blocks.block(b);
+                dev::mz_hits<K, SEC>(sh, t, seq, mask, base + dev::kMzBlock * b, lane, [&](uint32_t, uint32_t H) {
+                    count(p, H);
+                    later = H;
+                    p -= 32;
+                });
+            }
+            count(p, 0);
+        } else { // no start reaches the span
+            for (uint32_t q = sp.a + lane; q < sp.b; q += 32)
+                cov[sp.out + q] = 0;
         }
     }
 }
@@ -231,10 +283,10 @@ ibs_status coverage_device(ibs_table *t, const ibs_reference *ref, uint8_t *dCov
         k_map_spans_wide<<<grid, 256>>>(t->wide, ref->dSeq, ref->dMask, dSpans, spans.size(), dCov);
     else if (t->geom.format == FMT_B8X32)
         k_map_spans<FMT_B8X32><<<grid, 256>>>(v, ref->dSeq, ref->dMask, dSpans, spans.size(), dCov);
-    else if (t->geom.format == FMT_MZ8)
-        k_map_spans<FMT_MZ8><<<grid, 256>>>(v, ref->dSeq, ref->dMask, dSpans, spans.size(), dCov);
-    else if (t->geom.format == FMT_MZ6)
-        k_map_spans<FMT_MZ6><<<grid, 256>>>(v, ref->dSeq, ref->dMask, dSpans, spans.size(), dCov);
+    else if (is_mz(t->geom.format))
+        with_mz_table(t->geom, [&](auto K, auto SEC) {
+            k_map_spans_mz<K.value, SEC.value><<<grid, 256>>>(v, ref->dSeq, ref->dMask, dSpans, spans.size(), dCov);
+        });
     else
         k_map_spans<FMT_B6X40><<<grid, 256>>>(v, ref->dSeq, ref->dMask, dSpans, spans.size(), dCov);
     IBS_LAUNCHED();
