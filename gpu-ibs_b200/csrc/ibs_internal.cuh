@@ -234,6 +234,47 @@ struct WinDesc {
     uint32_t pad;
 };
 
+#if defined(__CUDACC__)
+namespace dev {
+// A window's row from its n span summaries, by one warp: each lane combines a
+// run of consecutive summaries, and a shuffle tree the 32 runs in order. (One
+// thread a window took 20 us for the 25 spans of a 50 kbp window, each load
+// waiting for the one before; small references have 200 shorter spans.)
+__device__ __forceinline__ void finish_window(const WinDesc &w, const SegStats *__restrict__ spans, uint32_t n, int k,
+                                              uint32_t lane, ibs_window *__restrict__ out)
+{
+    const uint32_t run = (n + 31) / 32, a = min(lane * run, n), b = min(a + run, n);
+    SegStats acc = seg_empty();
+    for (uint32_t s = a; s < b; ++s)
+        acc = seg_combine(acc, spans[s], k);
+#pragma unroll
+    for (uint32_t off = 1; off < 32; off <<= 1) {
+        SegStats o;
+        o.total = __shfl_down_sync(0xffffffffu, acc.total, off);
+        o.obs = __shfl_down_sync(0xffffffffu, acc.obs, off);
+        o.lead = __shfl_down_sync(0xffffffffu, acc.lead, off);
+        o.trail = __shfl_down_sync(0xffffffffu, acc.trail, off);
+        o.gaps = __shfl_down_sync(0xffffffffu, acc.gaps, off);
+        o.dist = __shfl_down_sync(0xffffffffu, acc.dist, off);
+        o.pad = 0;
+        acc = seg_combine(acc, o, k); // right for lanes that are multiples of 2 off
+    }
+    if (lane == 0) {
+        WindowRow row;
+        seg_finish(acc, k, row);
+        ibs_window o;
+        o.start = w.start;
+        o.end = w.end;
+        o.total_kmers = row.total_kmers;
+        o.observed_kmers = row.observed_kmers;
+        o.variations = row.variations;
+        o.kmer_distance = row.kmer_distance;
+        *out = o;
+    }
+}
+} // namespace dev
+#endif
+
 // Windows, spans and scratch of one (reference, W, k, span length) plan.
 struct ScanPlan {
     uint32_t W = 0, k = 0, spanLen = 0;
@@ -245,6 +286,12 @@ struct ScanPlan {
     SegStats *dSpans = nullptr;   // scratch: one summary per span
     void release();
 };
+
+// Positions per span for a reference (or a group of its windows) of `bases`:
+// the tuned length, or less where that would leave the GPU's warps without a
+// span. 1 Mbp in spans of 2048 is 490 warps on 32 of 148 SMs (51 us), in spans
+// of 256 3900 warps.
+uint32_t span_length(uint64_t bases, uint32_t tuned);
 
 // Build the plan's host arrays for contigs `lens` starting at packed
 // offsets `baseOff`.

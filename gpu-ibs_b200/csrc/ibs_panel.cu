@@ -376,29 +376,18 @@ __global__ void __launch_bounds__(256, 3) k_panel_spans_mz(const __grid_constant
     }
 }
 
-__global__ void k_panel_finalize(const WinDesc *__restrict__ win, const uint32_t *__restrict__ span0,
-                                 uint64_t nWin, uint64_t nSpans, uint32_t nSamples,
-                                 const SegStats *__restrict__ spans, int k, ibs_window *__restrict__ rows)
+__global__ void __launch_bounds__(256) k_panel_finalize(const WinDesc *__restrict__ win,
+                                                        const uint32_t *__restrict__ span0, uint64_t nWin,
+                                                        uint64_t nSpans, uint32_t nSamples,
+                                                        const SegStats *__restrict__ spans, int k,
+                                                        ibs_window *__restrict__ rows)
 {
-    const uint64_t total = nWin * nSamples;
-    for (uint64_t x = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; x < total;
-         x += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t total = nWin * nSamples, nWarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    for (uint64_t x = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; x < total; x += nWarps) {
         const uint64_t smp = x / nWin, w = x - smp * nWin;
-        SegStats acc = seg_empty();
-        for (uint32_t s = span0[w]; s < span0[w + 1]; ++s)
-            acc = seg_combine(acc, spans[smp * nSpans + s], k);
-        WindowRow row;
-        row.start = win[w].start;
-        row.end = win[w].end;
-        seg_finish(acc, k, row);
-        ibs_window o;
-        o.start = row.start;
-        o.end = row.end;
-        o.total_kmers = row.total_kmers;
-        o.observed_kmers = row.observed_kmers;
-        o.variations = row.variations;
-        o.kmer_distance = row.kmer_distance;
-        rows[x] = o;
+        const uint32_t s0 = span0[w];
+        dev::finish_window(win[w], spans + smp * nSpans + s0, span0[w + 1] - s0, k, lane, rows + x);
     }
 }
 
@@ -740,7 +729,10 @@ static uint32_t pass_count(const ibs_panel_table *p)
 // Plan and scratch of (reference, W) for the panel scan.
 static ibs_status panel_plan(ibs_panel_table *p, const ibs_reference *ref, uint32_t W)
 {
-    const uint32_t spanLen = tuning().panel_span_len;
+    uint64_t bases = 0;
+    for (uint64_t l : ref->lens)
+        bases += l;
+    const uint32_t spanLen = span_length(bases, tuning().panel_span_len);
     if (p->planRef == ref && p->plan.W == W && p->plan.dWin && p->planLens == ref->lens &&
         p->plan.spanLen == spanLen && (pass_count(p) <= 1 || p->dMasks))
         return IBS_OK;
@@ -822,7 +814,7 @@ static ibs_status panel_enqueue(ibs_panel_table *p, const ibs_reference *ref, ib
             return s;
     }
     if (pl.nWin && p->nSamples) {
-        k_panel_finalize<<<grid_for(pl.nWin * p->nSamples), 256, 0, st>>>(
+        k_panel_finalize<<<grid_for(pl.nWin * p->nSamples * 32), 256, 0, st>>>(
             pl.dWin, pl.dSpan0, pl.nWin, pl.nSpans, p->nSamples, p->dSpans, (int)p->geom.k, rowsDev);
         IBS_LAUNCHED();
     }

@@ -104,13 +104,10 @@ __global__ void __launch_bounds__(512) k_scan_spans(TableView t, const uint64_t 
                 const uint64_t h = perm_hash(code[b], t.g.bits);
                 const uint64_t r = bucket_of(h, t.g);
                 fp[b] = fp_of(h, t.g);
-                if (valid[b]) {
-                    v0[b] = __ldg(t.buckets + 2 * r);
-                    v1[b] = __ldg(t.buckets + 2 * r + 1);
-                } else {
-                    v0[b] = make_uint4(0, 0, 0, 0);
-                    v1[b] = make_uint4(0, 0, 0, 0);
-                }
+                v0[b] = make_uint4(0, 0, 0, 0);
+                v1[b] = make_uint4(0, 0, 0, 0);
+                if (valid[b])
+                    load_sector(t.buckets + 2 * r, v0[b], v1[b]);
             }
             uint32_t V[NB], H[NB];
 #pragma unroll
@@ -208,27 +205,15 @@ __global__ void __launch_bounds__(kMzThreads, 3) k_scan_spans_mz(const __grid_co
     }
 }
 
-__global__ void k_finalize(const WinDesc *__restrict__ win, const uint32_t *__restrict__ span0,
-                           uint64_t nWin, const SegStats *__restrict__ spans, int k,
-                           ibs_window *__restrict__ rows)
+__global__ void __launch_bounds__(256) k_finalize(const WinDesc *__restrict__ win, const uint32_t *__restrict__ span0,
+                                                  uint64_t nWin, const SegStats *__restrict__ spans, int k,
+                                                  ibs_window *__restrict__ rows)
 {
-    for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < nWin;
-         w += (uint64_t)gridDim.x * blockDim.x) {
-        SegStats acc = seg_empty();
-        for (uint32_t s = span0[w]; s < span0[w + 1]; ++s)
-            acc = seg_combine(acc, spans[s], k);
-        WindowRow row;
-        row.start = win[w].start;
-        row.end = win[w].end;
-        seg_finish(acc, k, row);
-        ibs_window o;
-        o.start = row.start;
-        o.end = row.end;
-        o.total_kmers = row.total_kmers;
-        o.observed_kmers = row.observed_kmers;
-        o.variations = row.variations;
-        o.kmer_distance = row.kmer_distance;
-        rows[w] = o;
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t nWarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    for (uint64_t w = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; w < nWin; w += nWarps) {
+        const uint32_t s0 = span0[w];
+        dev::finish_window(win[w], spans + s0, span0[w + 1] - s0, k, lane, rows + w);
     }
 }
 
@@ -252,6 +237,16 @@ void ScanPlan::release()
     nWin = nSpans = 0;
     win.clear();
     span0.clear();
+}
+
+// Below 128 positions a span has less than one block of the minimizer-line
+// scan; 24 warps a SM are what the scan kernels keep resident.
+uint32_t span_length(uint64_t bases, uint32_t tuned)
+{
+    const uint64_t warps = (uint64_t)sm_count() * 24;
+    while (tuned >= 256 && tuned % 256 == 0 && bases / tuned < warps)
+        tuned /= 2;
+    return tuned;
 }
 
 void plan_windows(ScanPlan &p, const std::vector<uint64_t> &lens,
@@ -369,7 +364,7 @@ static ibs_status launch_finalize_with(const ScanPlan &p, uint32_t k, const SegS
     if (!p.nWin)
         return IBS_OK;
     const int threads = 256;
-    const uint64_t want = (p.nWin + threads - 1) / threads;
+    const uint64_t want = (p.nWin * 32 + threads - 1) / threads;
     const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>(want, (uint64_t)sm_count() * 8));
     k_finalize<<<grid, threads, 0, st>>>(p.dWin, p.dSpan0, p.nWin, dSpans, (int)k, dRows);
     IBS_LAUNCHED();
@@ -706,7 +701,10 @@ extern "C" void ibs_reference_free(ibs_reference *r)
 static ibs_status ensure_plan(ibs_reference *r, uint32_t W, uint32_t k)
 {
     ScanPlan &p = r->plan;
-    const uint32_t spanLen = tuning().span_len;
+    uint64_t bases = 0;
+    for (uint64_t l : r->lens)
+        bases += l;
+    const uint32_t spanLen = span_length(bases, tuning().span_len);
     if (p.dWin && p.W == W && p.k == k && p.spanLen == spanLen)
         return IBS_OK;
     IBS_CUDA(cudaStreamSynchronize(r->stream), "plan sync");
@@ -963,7 +961,8 @@ extern "C" ibs_status ibs_scan_packed(ibs_table *t, const uint64_t *seq2bit,
     packed_offsets(lens, n, off, seqWords, maskWords);
     std::vector<uint64_t> lv(lens, lens + n);
     ScanPlan &p = ws.plan;
-    plan_windows(p, lv, off, W, k, tuning().span_len);
+    // the windows go in groups, the first a 128th of the reference
+    plan_windows(p, lv, off, W, k, span_length((seqWords - 1) * 32 / 8, tuning().span_len));
     if (p.nSpans > ws.spansCap || !p.dSpans) {
         cudaFree(p.dSpans);
         p.dSpans = nullptr;
