@@ -20,15 +20,18 @@ constexpr uint64_t kStashProbe = 64;
 // keys of one minimizer crowd its line, so the load stays below the hash
 // sectors' 3)
 constexpr double kPmKeysPerSector = 1.5;
+constexpr double kPm6KeysPerSector = 1.2; // the same share of a sector's four slots
 constexpr uint64_t kBuildChunk = 1ull << 27; // keys per build step (1 GiB of scratch each way)
 
-// Slot of fingerprint fp among sector w's first count slots, or -1.
-__device__ __forceinline__ int find_slot(const uint32_t *w, uint32_t fp)
+// Slot of fingerprint (or slot value) fp among sector w's first count slots,
+// or -1. wide: four 40-bit slot values (PM6).
+__device__ __forceinline__ int find_slot(const uint32_t *w, uint64_t fp, bool wide)
 {
-    const uint32_t cnt = (w[7] >> 16) & 0xff;
+    const uint32_t cnt = (w[7] >> 16) & 0xff, slots = wide ? kSlots6 : kSlots;
+    const uint32_t hi = wide ? (uint32_t)(fp >> 8) : (uint32_t)fp;
     int slot = -1;
-    for (uint32_t j = 0; j < cnt && j < kSlots; ++j)
-        if (w[j] == fp)
+    for (uint32_t j = 0; j < cnt && j < slots; ++j)
+        if (w[j] == hi && (!wide || ((w[4] >> (8 * j)) & 0xffu) == ((uint32_t)fp & 0xffu)))
             slot = (int)j;
     return slot;
 }
@@ -55,14 +58,15 @@ __device__ __forceinline__ bool stash_or(const View &t, unsigned long long *stas
     return false;
 }
 
-// Claims a free slot of sector w (bumps its count byte below kSlots) and
-// fills it with fp and the sample bit; false when the sector is full.
-__device__ __forceinline__ bool claim_slot(uint32_t *w, uint32_t fp, uint32_t bit)
+// Claims a free slot of sector w (bumps its count byte below the slots it has)
+// and fills it with fp and the sample bit; false when the sector is full.
+__device__ __forceinline__ bool claim_slot(uint32_t *w, uint64_t fp, uint32_t bit, bool wide)
 {
-    uint32_t old = w[7], slot = kSlots;
+    const uint32_t slots = wide ? kSlots6 : kSlots;
+    uint32_t old = w[7], slot = slots;
     for (int tries = 0; tries < 1 << 20; ++tries) {
         const uint32_t cnt = (old >> 16) & 0xff;
-        if (cnt >= kSlots)
+        if (cnt >= slots)
             break;
         const uint32_t seen = atomicCAS(w + 7, old, old + (1u << 16));
         if (seen == old) {
@@ -71,9 +75,11 @@ __device__ __forceinline__ bool claim_slot(uint32_t *w, uint32_t fp, uint32_t bi
         }
         old = seen;
     }
-    if (slot >= kSlots)
+    if (slot >= slots)
         return false;
-    w[slot] = fp;
+    w[slot] = wide ? (uint32_t)(fp >> 8) : (uint32_t)fp;
+    if (wide)
+        atomicOr(w + 4, ((uint32_t)fp & 0xffu) << (8 * slot));
     atomicOr(w + 5 + slot / 2, (1u << bit) << (16 * (slot & 1)));
     return true;
 }
@@ -89,11 +95,11 @@ __global__ void k_find(View t, uint32_t *words, unsigned long long *stashWords, 
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     const uint64_t iters = (n + stride - 1) / stride;
-    const bool pm = t.g.format == FMT_PANEL_MZ;
+    const bool pm = is_joint_mz(t.g.format), wide = t.g.format == FMT_PANEL_MZ6;
     for (uint64_t it = 0; it < iters; ++it) {
         const uint64_t i = it * stride + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-        uint64_t code = 0, r[2];
-        uint32_t fp[2], places = 0, turns = 0;
+        uint64_t code = 0, r[2], fp[2];
+        uint32_t places = 0, turns = 0;
         if (i < n) {
             code = codes[i];
             places = joint_places(t, code, r, fp);
@@ -105,14 +111,14 @@ __global__ void k_find(View t, uint32_t *words, unsigned long long *stashWords, 
                 miss = !stash_or(t, stashWords, code, bit);
             } else if (a < turns) {
                 const uint64_t ra = a ? r[1] : r[0];
-                const uint32_t fa = a ? fp[1] : fp[0];
+                const uint64_t fa = a ? fp[1] : fp[0];
                 uint32_t *w = words + 8 * ra;
                 const uint32_t flags = w[7];
-                int slot = find_slot(w, fa);
+                int slot = find_slot(w, fa, wide);
                 uint32_t *where = w;
                 for (uint32_t d = 1; d < 4 && slot < 0 && pm && (flags & (d == 1 ? kPartnerFlag : kLineFlag)); ++d) {
                     where = words + 8 * (ra ^ d);
-                    slot = find_slot(where, fa);
+                    slot = find_slot(where, fa, wide);
                 }
                 if (slot >= 0)
                     atomicOr(where + 5 + slot / 2, (1u << bit) << (16 * (slot & 1)));
@@ -136,27 +142,26 @@ __global__ void k_find(View t, uint32_t *words, unsigned long long *stashWords, 
 __global__ void k_insert(View t, uint32_t *words, unsigned long long *stashWords, const uint64_t *codes,
                          uint64_t n, uint32_t bit, uint64_t *failed, unsigned long long *nFailed)
 {
-    const bool pm = t.g.format == FMT_PANEL_MZ;
+    const bool pm = is_joint_mz(t.g.format), wide = t.g.format == FMT_PANEL_MZ6;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
          i += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t entered = codes[i];
         const uint64_t code = pm ? entered & ~(mz::kSecondPlace | mz::kNoPlace) : entered;
         if (!pm || !(entered & mz::kNoPlace)) {
-            uint64_t rr[2];
-            uint32_t ff[2];
+            uint64_t rr[2], ff[2];
             joint_places(t, code, rr, ff);
             const bool second = pm && (entered & mz::kSecondPlace);
             const uint64_t r = second ? rr[1] : rr[0];
-            const uint32_t fp = second ? ff[1] : ff[0];
+            const uint64_t fp = second ? ff[1] : ff[0];
             uint32_t *w = words + 8 * r;
-            if (claim_slot(w, fp, bit))
+            if (claim_slot(w, fp, bit, wide))
                 continue;
             if (pm) { // the line's other sectors, flagged on the home sector
                 atomicOr(w + 7, kPartnerFlag);
-                bool claimed = claim_slot(words + 8 * (r ^ 1), fp, bit);
+                bool claimed = claim_slot(words + 8 * (r ^ 1), fp, bit, wide);
                 if (!claimed) {
                     atomicOr(w + 7, kLineFlag);
-                    claimed = claim_slot(words + 8 * (r ^ 2), fp, bit) || claim_slot(words + 8 * (r ^ 3), fp, bit);
+                    claimed = claim_slot(words + 8 * (r ^ 2), fp, bit, wide) || claim_slot(words + 8 * (r ^ 3), fp, bit, wide);
                 }
                 if (claimed)
                     continue;
@@ -323,7 +328,7 @@ __global__ void __launch_bounds__(256) k_panel_spans(View t, const uint64_t *__r
     }
 }
 
-// The minimizer-line tables (PM), k fixed at compile time: located 128
+// The minimizer-line tables (PM, PM6), k fixed at compile time: located 128
 // positions at a time as the single-sample scan (mz_scan.cuh), one sector
 // load a position, then kScan's statistics or kMaskPass's masks.
 template <uint32_t K, int MODE>
@@ -336,8 +341,9 @@ __global__ void __launch_bounds__(256, 3) k_panel_spans_mz(const __grid_constant
                                                            SegStats *__restrict__ out, uint16_t *__restrict__ masks,
                                                            uint64_t bLo, uint64_t bHi, bool firstPass)
 {
-    __shared__ dev::MzShared<FMT_B8X32> shared[8];
-    dev::MzShared<FMT_B8X32> *sh = &shared[threadIdx.x >> 5];
+    constexpr uint32_t SEC = joint_mz_slots(K);
+    __shared__ dev::MzShared<SEC> shared[8];
+    dev::MzShared<SEC> *sh = &shared[threadIdx.x >> 5];
     const uint32_t lane = dev::lane_id();
     for (;;) {
         unsigned long long s = 0;
@@ -351,7 +357,7 @@ __global__ void __launch_bounds__(256, 3) k_panel_spans_mz(const __grid_constant
         const uint32_t nPos = win[w].nPos;
         const uint32_t p0 = (uint32_t)(s - __ldg(span0 + w)) * spanLen;
         const uint32_t n = min(spanLen, nPos - p0);
-        dev::MzWarp<K, FMT_B8X32> warp(sh, t.g, seq, mask, base + p0, n, base + nPos - 1 + (K - 1), lane);
+        dev::MzWarp<K, SEC> warp(sh, t.g, seq, mask, base + p0, n, base + nPos - 1 + (K - 1), lane);
         JointFold fold(lane);
         warp.start();
         for (int b = warp.blocks() - 1; b >= 0; --b) {
@@ -483,6 +489,20 @@ extern "C" ibs_status ibs_panel_table_create(uint32_t k, uint64_t expected_keys,
     const uint64_t pmLines = (uint64_t)((double)expected_keys / lamPm / mz::kSectorsPerLine) + 1;
     if (fmt == 0 && k >= 16 && k <= 27 && pmLines >= pmMinLines && pmLines < (1ull << 31))
         fmt = FMT_PANEL_MZ; // the default where its minimum size does not oversize the table
+    // k = 28 .. 31, at the default load: minimizer lines of 40-bit slots where
+    // their minimum size does not oversize the table, it stays within one
+    // bucket-range pass and there is room for it. (Hash sectors cost a random
+    // line a position: 200 Mbp against 16 samples 4.5 ms, on lines 2.2 ms. But
+    // they take half the memory, and past 48 GiB random lines get slow. A caller
+    // who gives a load has planned for the hash sectors'.)
+    const uint64_t pm6Lines = (uint64_t)((double)expected_keys / kPm6KeysPerSector / mz::kSectorsPerLine) + 1;
+    if (fmt == 0 && k >= 28 && k <= 31 && !(opts && opts->keys_per_bucket > 0) && pm6Lines >= 1ull << (2 * k - 37) &&
+        pm6Lines * 128 <= 48ull << 30) {
+        size_t freeBytes = 0, totalBytes = 0;
+        IBS_CUDA(cudaMemGetInfo(&freeBytes, &totalBytes), "cudaMemGetInfo");
+        if (pm6Lines * 128 + pm6Lines * 16 <= freeBytes)
+            fmt = FMT_PANEL_MZ6;
+    }
     if (fmt == 0)
         fmt = FMT_PANEL;
     g.format = fmt;
@@ -494,6 +514,11 @@ extern "C" ibs_status ibs_panel_table_create(uint32_t k, uint64_t expected_keys,
         nb = nLines * mz::kSectorsPerLine;
         g.nBuckets = nb;
         g.fpBits = 2 * mz::m_of(k) - (uint32_t)(63 - __builtin_clzll(nLines));
+    } else if (fmt == FMT_PANEL_MZ6) {
+        lam = kPm6KeysPerSector;
+        nb = pm6Lines * mz::kSectorsPerLine;
+        g.nBuckets = nb;
+        g.fpBits = 2 * mz::m_of(k) - (uint32_t)(63 - __builtin_clzll(pm6Lines));
     } else {
         lam = (opts && opts->keys_per_bucket > 0) ? opts->keys_per_bucket : tuning().panel_keys_per_bucket;
         nb = (uint64_t)((double)expected_keys / lam) + 1;
@@ -509,8 +534,9 @@ extern "C" ibs_status ibs_panel_table_create(uint32_t k, uint64_t expected_keys,
     // minimizer lines: the keys of one minimizer crowd its line, so far more
     // than a Poisson share of them overflows (about 2% at 1.5 keys per
     // sector, 10% at 3); sized here for twice that, the stash grows if needed
-    const double over = fmt == FMT_PANEL_MZ
-                            ? (double)expected_keys * std::min(0.5, 0.04 * lam / 1.5 * lam / 1.5 + 0.01)
+    const double most = fmt == FMT_PANEL_MZ6 ? kPm6KeysPerSector : kPmKeysPerSector;
+    const double over = is_joint_mz(fmt)
+                            ? (double)expected_keys * std::min(0.5, 0.04 * lam / most * lam / most + 0.01)
                             : (double)expected_keys * overflow_fraction((double)expected_keys / (double)nb);
     p->stashBuckets = next_pow2(std::max<uint64_t>(1u << 12, (uint64_t)(over * 0.75) + 1));
     g.stashBuckets = p->stashBuckets;
@@ -583,7 +609,7 @@ static ibs_status panel_add_device_codes(ibs_panel_table *p, const uint64_t *dCo
     // keys go in chunks, so the build's scratch stays small next to the table
     const uint64_t chunk = std::max<uint64_t>(1, std::min<uint64_t>(n, kBuildChunk));
     uint64_t *pending = nullptr, *failed = nullptr;
-    const uint64_t places = p->geom.format == FMT_PANEL_MZ ? 2 : 1; // most places a key has
+    const uint64_t places = is_joint_mz(p->geom.format) ? 2 : 1; // most places a key has
     IBS_CUDA(cudaMalloc(&pending, chunk * places * 8), "panel pending alloc");
     std::unique_ptr<uint64_t, cudaError_t (*)(void *)> g1(pending, cudaFree);
     IBS_CUDA(cudaMalloc(&failed, chunk * places * 8), "panel pending alloc");
@@ -787,17 +813,17 @@ static ibs_status enqueue_spans(ibs_panel_table *p, const ibs_reference *ref, ui
     };
     ibs_status s = IBS_OK;
     if (passes <= 1) {
-        if (p->geom.format != FMT_PANEL_MZ)
+        if (!is_joint_mz(p->geom.format))
             return go(k_panel_spans<NB, kScan>, 0, 0, false);
-        with_mz_k<16, 27>(p->geom.k, [&](auto K) { s = go(k_panel_spans_mz<K.value, kScan>, 0, 0, false); });
+        with_mz_k<16, 31>(p->geom.k, [&](auto K) { s = go(k_panel_spans_mz<K.value, kScan>, 0, 0, false); });
         return s;
     }
     for (uint32_t i = 0; i < passes && s == IBS_OK; ++i) {
         const uint64_t bLo = nb * i / passes, bHi = nb * (i + 1) / passes;
-        if (p->geom.format != FMT_PANEL_MZ)
+        if (!is_joint_mz(p->geom.format))
             s = go(k_panel_spans<NB, kMaskPass>, bLo, bHi, i == 0);
         else
-            with_mz_k<16, 27>(p->geom.k, [&](auto K) { s = go(k_panel_spans_mz<K.value, kMaskPass>, bLo, bHi, i == 0); });
+            with_mz_k<16, 31>(p->geom.k, [&](auto K) { s = go(k_panel_spans_mz<K.value, kMaskPass>, bLo, bHi, i == 0); });
     }
     return s == IBS_OK ? go(k_panel_spans<NB, kStats>, 0, 0, false) : s;
 }

@@ -186,12 +186,12 @@ __device__ __forceinline__ void serve_joint_item(const WorkItem &it, const panel
     const bool one = (want & (want - 1u)) == 0u; // warp-uniform
     const uint32_t j0 = __ffs(want) - 1;
     const uint32_t rank = __popc(want & ((1u << lane) - 1u));
-    if constexpr (K >= 16 && K <= 27) {
-        if (t.g.format == FMT_PANEL_MZ) {
-            auto *sh = reinterpret_cast<dev::MzShared<FMT_B8X32> *>(shared);
+    if constexpr (K >= 16 && K <= 31) {
+        if (t.g.format == panel::joint_mz_format(K)) {
+            constexpr uint32_t SEC = panel::joint_mz_slots(K);
+            auto *sh = reinterpret_cast<dev::MzShared<SEC> *>(shared);
             const uint64_t first = it.base + it.p0;
-            dev::MzWarp<K, FMT_B8X32> warp(sh, t.g, seq, mask, first, it.p1 - it.p0, it.base + it.p1 - 1 + (K - 1),
-                                           lane);
+            dev::MzWarp<K, SEC> warp(sh, t.g, seq, mask, first, it.p1 - it.p0, it.base + it.p1 - 1 + (K - 1), lane);
             dev::LaneFold<true> lone;
             panel::JointFold fold(lane);
             warp.start();

@@ -26,6 +26,11 @@
 // random ones. A full sector keeps further keys in its partner sector (index
 // ^ 1, the same line; flag bit 25 of byte 31's word), then in the line's
 // other two (bit 26) and then in the stash (bit 24).
+//
+// Format PM6 (FMT_PANEL_MZ6, 28 <= k <= 31): the same lines for 40-bit slot
+// values, four slots a sector: their high 32 bits in words 0-3, low bytes in
+// word 4, masks in words 5-6, count and flags in word 7 as above (at least
+// 2^(2k-37) lines).
 #pragma once
 
 #include "ibs_internal.cuh"
@@ -37,7 +42,11 @@ namespace ibs {
 namespace panel {
 
 constexpr uint32_t kMaxSamples = IBS_PANEL_MAX_SAMPLES;
-constexpr uint32_t kSlots = 5;
+constexpr uint32_t kSlots = 5, kSlots6 = 4;
+// The minimizer-line layout of a k, and the sector layout whose slot values it has.
+IBS_HD bool is_joint_mz(uint32_t fmt) { return fmt == FMT_PANEL_MZ || fmt == FMT_PANEL_MZ6; }
+constexpr uint32_t joint_mz_format(uint32_t k) { return k <= 27 ? FMT_PANEL_MZ : FMT_PANEL_MZ6; }
+constexpr uint32_t joint_mz_slots(uint32_t k) { return k <= 27 ? FMT_B8X32 : FMT_B6X40; }
 constexpr uint64_t kStashEmpty = ~0ull;
 constexpr uint32_t kStashFlag = 1u << 24;   // word 7: some key of this sector is in the stash
 constexpr uint32_t kPartnerFlag = 1u << 25; // word 7 (PM): some key of this sector is in its partner sector
@@ -78,6 +87,21 @@ __device__ __forceinline__ uint32_t sector_mask(const uint4 &v0, const uint4 &v1
     return m;
 }
 
+// The same of a minimizer line's sector, for a slot value of 32 (PM) or 40
+// bits (PM6: high holds its top byte).
+template <bool WIDE>
+__device__ __forceinline__ uint32_t line_sector_mask(const uint4 &v0, const uint4 &v1, uint32_t slot, uint32_t high)
+{
+    if (!WIDE)
+        return sector_mask(v0, v1, slot);
+    const uint32_t hi = __funnelshift_r(slot, high, 8), d = v1.x ^ ((slot & 0xffu) * 0x01010101u);
+    uint32_t m = v0.x == hi && !(d & 0x000000ffu) ? v1.y & 0xffffu : 0u;
+    m |= v0.y == hi && !(d & 0x0000ff00u) ? v1.y >> 16 : 0u;
+    m |= v0.z == hi && !(d & 0x00ff0000u) ? v1.z & 0xffffu : 0u;
+    m |= v0.w == hi && !(d & 0xff000000u) ? v1.z >> 16 : 0u;
+    return m;
+}
+
 // Sample mask of a k-mer given its bucket halves and fingerprint; bit 31
 // set = look in the stash.
 __device__ __forceinline__ uint32_t bucket_mask(const uint4 &v0, const uint4 &v1, uint32_t fp)
@@ -88,12 +112,17 @@ __device__ __forceinline__ uint32_t bucket_mask(const uint4 &v0, const uint4 &v1
     return m;
 }
 
-// PM: the mask of a k-mer that its home sector r does not hold, from the
-// line's other sectors as the home sector's flags say (the stash is next).
-__device__ __forceinline__ uint32_t pm_line_mask(const View &t, uint32_t flags, uint64_t r, uint32_t slot)
+// Minimizer lines: the mask of a k-mer that its home sector r does not hold,
+// from the line's other sectors as the home sector's flags say (the stash is
+// next).
+template <bool WIDE>
+__device__ __forceinline__ uint32_t pm_line_mask(const View &t, uint32_t flags, uint64_t r, uint32_t slot,
+                                                 uint32_t high)
 {
     uint32_t m = 0;
-    auto look = [&](uint64_t x) { return sector_mask(__ldg(t.buckets + 2 * x), __ldg(t.buckets + 2 * x + 1), slot); };
+    auto look = [&](uint64_t x) {
+        return line_sector_mask<WIDE>(__ldg(t.buckets + 2 * x), __ldg(t.buckets + 2 * x + 1), slot, high);
+    };
     if (flags & kPartnerFlag) {
         m = look(r ^ 1);
         if (!m && (flags & kLineFlag))
@@ -102,49 +131,53 @@ __device__ __forceinline__ uint32_t pm_line_mask(const View &t, uint32_t flags, 
     return m;
 }
 
-// Home sectors and stored fingerprints (P5x48) or slot values (PM) of a key;
+// Home sectors and stored fingerprints (P5x48) or slot values of a key;
 // returns how many places it has (mz::placements; none: the stash only).
-__device__ __forceinline__ uint32_t joint_places(const View &t, uint64_t code, uint64_t r[2], uint32_t fp[2])
+__device__ __forceinline__ uint32_t joint_places(const View &t, uint64_t code, uint64_t r[2], uint64_t fp[2])
 {
-    if (t.g.format == FMT_PANEL_MZ) {
-        uint64_t slot[2];
-        const uint32_t n = mz::placements(code, t.g, r, slot);
-        fp[0] = n ? (uint32_t)slot[0] : 0u;
-        fp[1] = n == 2 ? (uint32_t)slot[1] : 0u;
-        return n;
-    }
+    if (is_joint_mz(t.g.format))
+        return mz::placements(code, t.g, r, fp);
     const uint64_t h = perm_hash(code, t.g.bits);
     r[0] = bucket_of(h, t.g);
-    fp[0] = (uint32_t)fp_of(h, t.g);
+    fp[0] = fp_of(h, t.g);
     return 1;
+}
+
+template <bool WIDE>
+__device__ __forceinline__ uint32_t lookup_line_mask(const View &t, uint64_t code, uint64_t r, uint64_t fp)
+{
+    uint4 v0, v1;
+    load_sector(t.buckets + 2 * r, v0, v1);
+    uint32_t m = line_sector_mask<WIDE>(v0, v1, (uint32_t)fp, (uint32_t)(fp >> 32));
+    if (!m)
+        m = pm_line_mask<WIDE>(t, v1.w, r, (uint32_t)fp, (uint32_t)(fp >> 32));
+    return !m && (v1.w & kStashFlag) ? stash_mask(t, code) : m;
 }
 
 __device__ __forceinline__ uint32_t lookup_mask(const View &t, uint64_t code)
 {
-    uint64_t r[2];
-    uint32_t fp[2];
+    uint64_t r[2], fp[2];
     if (!joint_places(t, code, r, fp))
         return stash_mask(t, code);
+    if (t.g.format == FMT_PANEL_MZ)
+        return lookup_line_mask<false>(t, code, r[0], fp[0]);
+    if (t.g.format == FMT_PANEL_MZ6)
+        return lookup_line_mask<true>(t, code, r[0], fp[0]);
     uint4 v0, v1;
     load_sector(t.buckets + 2 * r[0], v0, v1);
-    if (t.g.format == FMT_PANEL_MZ) {
-        uint32_t m = sector_mask(v0, v1, fp[0]);
-        if (!m)
-            m = pm_line_mask(t, v1.w, r[0], fp[0]);
-        return !m && (v1.w & kStashFlag) ? stash_mask(t, code) : m;
-    }
-    const uint32_t m = bucket_mask(v0, v1, fp[0]);
+    const uint32_t m = bucket_mask(v0, v1, (uint32_t)fp[0]);
     return m & 0x80000000u ? stash_mask(t, code) : m;
 }
 
 // The same of the k-mer at packed base G, out of line (see dev::mz_elsewhere);
 // flags is the home sector's flag byte.
-static __device__ __noinline__ uint32_t elsewhere_mask(const View *t, const uint64_t *__restrict__ seq,
-                                                       const uint64_t *__restrict__ mask, uint64_t G, uint32_t k,
-                                                       uint32_t line, uint32_t slot, uint32_t flags)
+template <bool WIDE>
+__device__ __noinline__ uint32_t elsewhere_mask(const View *t, const uint64_t *__restrict__ seq,
+                                                const uint64_t *__restrict__ mask, uint64_t G, uint32_t k,
+                                                uint32_t line, uint32_t slot, uint32_t high, uint32_t flags)
 {
-    const uint32_t m =
-        pm_line_mask(*t, flags << 24, (uint64_t)line * mz::kSectorsPerLine + mz::sector_of(slot, 0), slot);
+    const uint32_t m = pm_line_mask<WIDE>(
+        *t, flags << 24, (uint64_t)line * mz::kSectorsPerLine + mz::sector_of(slot, high), slot, high);
     if (m || !((flags << 24) & kStashFlag))
         return m;
     bool acgt;
@@ -155,11 +188,12 @@ static __device__ __noinline__ uint32_t elsewhere_mask(const View *t, const uint
 // is position 32 i + lane's, valid[i] whether it has a k-mer. RANGE: sectors
 // outside [bLo, bHi) count as empty (they read sector bLo).
 template <uint32_t K, bool RANGE>
-__device__ __forceinline__ void mz_masks(const dev::MzShared<FMT_B8X32> *sh, const View &t,
+__device__ __forceinline__ void mz_masks(const dev::MzShared<joint_mz_slots(K)> *sh, const View &t,
                                          const uint64_t *__restrict__ seq, const uint64_t *__restrict__ mask,
                                          uint64_t blockBase, uint32_t lane, uint64_t bLo, uint64_t bHi,
                                          uint32_t (&m)[4], bool (&valid)[4])
 {
+    constexpr bool kWide = K > 27;
     uint32_t more = 0; // 3 bits a position: the flags of a full sector that does not hold it
     {
         dev::MzSectors s;
@@ -180,7 +214,7 @@ __device__ __forceinline__ void mz_masks(const dev::MzShared<FMT_B8X32> *sh, con
             valid[i] = s.valid(i);
             if (!RANGE)
                 mine[i] = valid[i];
-            m[i] = mine[i] ? sector_mask(s.v0[i], s.v1[i], s.slot[i]) : 0u;
+            m[i] = mine[i] ? line_sector_mask<kWide>(s.v0[i], s.v1[i], s.slot[i], s.high[i]) : 0u;
             if (mine[i] && !m[i])
                 more |= ((s.v1[i].w >> 24) & 7u) << (3 * i);
         }
@@ -189,8 +223,8 @@ __device__ __forceinline__ void mz_masks(const dev::MzShared<FMT_B8X32> *sh, con
         const int i = (__ffs(more) - 1) / 3;
         dev::MzSectors s;
         s.record(sh, 0, 32 * i + lane);
-        const uint32_t x = elsewhere_mask(&t, seq, mask, blockBase + 32 * i + lane, K, s.line[0], s.slot[0],
-                                          (more >> (3 * i)) & 7u);
+        const uint32_t x = elsewhere_mask<kWide>(&t, seq, mask, blockBase + 32 * i + lane, K, s.line[0], s.slot[0],
+                                                 s.high[0], (more >> (3 * i)) & 7u);
         m[0] = i == 0 ? x : m[0];
         m[1] = i == 1 ? x : m[1];
         m[2] = i == 2 ? x : m[2];

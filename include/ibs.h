@@ -265,7 +265,10 @@ ibs_status ibs_scan_panel(ibs_table *const *tables, uint32_t n_tables, ibs_refer
  * lines (16 <= k <= 27, at least 2^(2k-28) lines; consecutive positions
  * share 128-byte lines, a full sector spills into the line's others, then
  * the stash; default load 1.5 keys per sector); 0 = 7 where it applies and its
- * minimum size does not oversize the table, else 3. opts->keys_per_bucket: keys
+ * minimum size does not oversize the table, for 28 <= k <= 31 the same with
+ * 40-bit slots (reported as format 9; four slots a sector, at least 2^(2k-37)
+ * lines, at the default load, up to 48 GiB and where the device has room), else
+ * 3. opts->keys_per_bucket: keys
  * per sector (0 = the tuned panel_keys_per_bucket for 3, 1.5 for 7). Samples are added one at a
  * time (sample i = the i-th call); rows are sample-major:
  * rows[i * n_windows + w]. The scan is a persistent kernel over a work queue

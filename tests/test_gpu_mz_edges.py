@@ -114,3 +114,40 @@ def test_noalloc_edges(k):
             ib.scan_noalloc(t, dseq, dmask, lens, W, rows, len(want), torch.cuda.current_stream().cuda_stream)
             torch.cuda.synchronize()
             assert np.array_equal(rows.cpu().numpy(), want.view(np.int32).reshape(-1, 6)), (k, fmt, W)
+
+
+@pytest.mark.parametrize("k", [28, 29, 30, 31])
+@pytest.mark.parametrize("passes", [1, 3])
+def test_joint_lines_of_long_k(k, passes):
+    """Joint tables of k = 28 .. 31 that expect enough keys take minimizer lines
+    of 40-bit slots: masks and rows as the hash sectors', in one pass and in
+    bucket ranges."""
+    seqs, codes = _world(k)
+    rng = np.random.default_rng(k)
+    share = [codes[rng.random(len(codes)) < 0.2 + 0.05 * i] for i in range(16)]
+    ref = ib.Reference(*ib.pack_ascii(seqs))
+    many = int((1 << (2 * k - 37)) * 4 * 1.2) + 100_000
+    t = ib.PanelTable(k, many)
+    h = ib.PanelTable(k, 16, force_format=3) if k < 30 else None  # 2^(2k - 32) sectors at least
+    for c in share:
+        t.add_codes(c, len(c), on_device=False)
+        if h is not None:
+            h.add_codes(c, len(c), on_device=False)
+    assert t.info()[0].format not in (3, 7)
+    want = sum(np.isin(codes, c).astype(np.uint32) << np.uint32(i) for i, c in enumerate(share))
+    assert np.array_equal(t.probe(codes), want)
+    tune = ib.get_tuning()
+    kept = tune.panel_pass_mb
+    if passes > 1:
+        tune.panel_pass_mb = max(1, int(t.info()[0].n_buckets * 32 / passes / (1 << 20)) + 1)
+        ib.set_tuning(tune)
+    try:
+        for W in (k + 1, k + 128, 1000, 20_000):
+            rows = t.scan(ref, W)
+            if h is not None:
+                assert np.array_equal(rows, h.scan(ref, W)), (k, W)
+            one = ib.Table.from_codes(share[7], len(share[7]), k, on_device=False, force_format=5)
+            assert np.array_equal(rows[7], ib.scan(one, ref, W)), (k, W)
+    finally:
+        tune.panel_pass_mb = kept if kept else 0xFFFFFFFF
+        ib.set_tuning(tune)
