@@ -337,4 +337,16 @@ IBS_HD uint64_t windows_in_contig(uint64_t len, uint32_t W, uint32_t k)
 // ---------------------------------------------------------------------------
 IBS_HD uint64_t round_up64(uint64_t x) { return (x + 63) & ~63ull; }
 
+#if defined(__CUDACC__)
+// A 32-byte sector in one load (two 16-byte loads ask the L1 twice; with many
+// probes in flight random sectors came at 25 to 34 G/s so, at 36.4 G/s with
+// one load each, whatever is in flight).
+__device__ __forceinline__ void load_sector(const uint4 *p, uint4 &a, uint4 &b)
+{
+    asm volatile("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
+                 : "l"(p));
+}
+#endif
+
 } // namespace ibs

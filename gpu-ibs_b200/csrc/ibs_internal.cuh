@@ -132,16 +132,6 @@ __device__ __forceinline__ uint32_t bucket_match(const uint4 &v0, const uint4 &v
     }
 }
 
-// A 32-byte sector in one load (two 16-byte loads ask the L1 twice; with many
-// probes in flight random sectors came at 25 to 34 G/s so, at 36.4 G/s with
-// one load each, whatever is in flight).
-__device__ __forceinline__ void load_sector(const uint4 *p, uint4 &a, uint4 &b)
-{
-    asm volatile("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
-                 : "l"(p));
-}
-
 // Whether a minimizer line's sector holds a slot value. B6x40: each slot's
 // 32-bit half by one comparison and its byte by one masked difference; the
 // slots past the count hold zeros, which only a slot value of zero can match.

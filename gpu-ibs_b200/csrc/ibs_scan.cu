@@ -130,15 +130,17 @@ __global__ void __launch_bounds__(512) k_scan_spans(TableView t, const uint64_t 
 
 // The scan over a wide-key table (33 <= k <= 64, format FMT_WIDE): the span
 // loop of k_scan_spans with each lane's k-mer read as a 128-bit canonical
-// code from three packed words and the warp's 32 codes looked up together,
-// 8 lanes reading each 128-byte line (wide::lookup_warp).
+// code from three packed words, and each key's home half line
+// read by two lanes (wide::PairProbe): 42 G probes/s over 0.24 GB of
+// table, 32 over 1.9 GB (eight lanes a line, which reads every line whole: 23
+// and 27; two or four blocks of 32 positions in flight a lane: 32 and 23).
 // Restates the reference's string path for these k: canonical k-mer strings
 // of the window (getCanonicalKmersLegacy, src/Utils.hpp:102-125: toupper,
 // k-mers with a non-ACGT byte skipped, the smaller of the k-mer and its
 // reverse complement) each looked up in the database
 // (getStatsFromSequenceLegacy, src/KmerDatabase.hpp:675-708), with the same
 // statistics fold.
-__global__ void __launch_bounds__(256) k_scan_spans_wide(wide::View t, const uint64_t *__restrict__ seq,
+__global__ void __launch_bounds__(256) k_scan_spans_wide(const __grid_constant__ wide::View t, const uint64_t *__restrict__ seq,
                                                          const uint64_t *__restrict__ mask,
                                                          const WinDesc *__restrict__ win,
                                                          const uint32_t *__restrict__ span0, uint32_t nWin,
@@ -161,12 +163,17 @@ __global__ void __launch_bounds__(256) k_scan_spans_wide(wide::View t, const uin
             const bool inSpan = q < p1;
             // lanes past the span read a position inside it and are masked out
             const uint64_t G = base + (inSpan ? q : p0);
-            bool acgt;
+            bool acgt, hit, full;
             uint64_t lo, hi;
             wide::canonical_at(seq, mask, G, k, acgt, lo, hi);
             const bool valid = inSpan && acgt;
-            const bool hit = wide::lookup_warp(t, lo, hi, valid, lane);
-            fold.push(__ballot_sync(FULL, valid), __ballot_sync(FULL, hit), lane, (int)k);
+            const uint64_t home = wide::home_of(lo, hi, 0, t.lines[0]);
+            wide::PairProbe x;
+            x.load(t, lo, hi, home, lane);
+            x.result(lane, hit, full);
+            if (valid && !hit && full)
+                hit = wide::lookup_rest(t, lo, hi, home);
+            fold.push(__ballot_sync(FULL, valid), __ballot_sync(FULL, valid && hit), lane, (int)k);
         }
         const SegStats acc = fold.finish((int)k);
         if (lane == 0)

@@ -4,11 +4,10 @@
 // The reference has no device table for these k: its string path looks each
 // canonical k-mer string up in the KMC database on the host
 // (getStatsFromSequenceLegacy, src/KmerDatabase.hpp:675-708; CKmerAPI::
-// from_string + CKMCFile::IsKmer). The build here is a counting placement:
-// per level, every key counts its line, lines with more than 8 keys send the
-// surplus to the next level's input, and every key then claims a slot of its
-// line in arrival order (the first 8 of a line stay; which 8 does not
-// matter to membership).
+// from_string + CKMCFile::IsKmer). The build here is one pass a level: every
+// key claims the next free slot of its home half line, then of the line's
+// other half (a 128-bit compare-and-swap), and a key whose line is full goes
+// to the next level's input (which 8 stay does not matter to membership).
 #include "ibs_internal.cuh"
 
 #include <algorithm>
@@ -25,54 +24,43 @@ using wide::kSlots;
 
 __device__ __forceinline__ bool is_empty_key(const ulonglong2 &v) { return v.x == kEmpty && v.y == kEmpty; }
 
-__global__ void k_wcount(const ulonglong2 *__restrict__ keys, uint64_t n, uint32_t level, uint64_t lines,
-                         uint32_t *__restrict__ cnt)
+// Puts v in an empty slot; false when another key has it.
+__device__ __forceinline__ bool claim_slot(ulonglong2 *slot, const ulonglong2 &v)
 {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
-         i += (uint64_t)gridDim.x * blockDim.x) {
-        const ulonglong2 v = keys[i];
-        if (!is_empty_key(v))
-            atomicAdd(cnt + wide::line_of(v.x, v.y, level, lines), 1u);
-    }
-}
-
-// Keys beyond kSlots per line (the next level's input), summed; resets the
-// counters for the placement pass.
-__global__ void k_wover(uint32_t *__restrict__ cnt, uint64_t lines, unsigned long long *__restrict__ over)
-{
-    unsigned long long local = 0;
-    for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < lines;
-         r += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t c = cnt[r];
-        if (c > kSlots)
-            local += c - kSlots;
-        cnt[r] = 0;
-    }
-    for (int o = 16; o; o >>= 1)
-        local += __shfl_xor_sync(0xffffffffu, local, o);
-    if ((threadIdx.x & 31) == 0 && local)
-        atomicAdd(over, local);
+    unsigned long long lo, hi;
+    asm volatile("{\n\t"
+                 ".reg .b128 old, cmp, val;\n\t"
+                 "mov.b128 cmp, {%4, %4};\n\t"
+                 "mov.b128 val, {%2, %3};\n\t"
+                 "atom.global.cas.b128 old, [%5], cmp, val;\n\t"
+                 "mov.b128 {%0, %1}, old;\n\t"
+                 "}"
+                 : "=l"(lo), "=l"(hi)
+                 : "l"(v.x), "l"(v.y), "l"(kEmpty), "l"(slot)
+                 : "memory");
+    return lo == kEmpty && hi == kEmpty;
 }
 
 __global__ void k_wplace(const ulonglong2 *__restrict__ keys, uint64_t n, uint32_t level, uint64_t lines,
-                         uint32_t *__restrict__ cnt, ulonglong2 *__restrict__ slots, ulonglong2 *__restrict__ next,
-                         unsigned long long *__restrict__ nextN, uint64_t nextCap, int *__restrict__ err)
+                         ulonglong2 *__restrict__ slots, ulonglong2 *__restrict__ next,
+                         unsigned long long *__restrict__ nextN, uint64_t nextCap)
 {
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
          i += (uint64_t)gridDim.x * blockDim.x) {
         const ulonglong2 v = keys[i];
         if (is_empty_key(v))
             continue;
-        const uint64_t r = wide::line_of(v.x, v.y, level, lines);
-        const uint32_t s = atomicAdd(cnt + r, 1u);
-        if (s < kSlots) {
-            slots[r * kSlots + s] = v;
-        } else {
+        const uint64_t home = wide::home_of(v.x, v.y, level, lines);
+        bool placed = false;
+        for (uint32_t j = 0; j < kSlots && !placed; ++j) { // the home half's slots, then the other's
+            ulonglong2 *slot = slots + (j < kSlots / 2 ? home + j : (home ^ (kSlots / 2)) + (j - kSlots / 2));
+            const ulonglong2 old = __ldcg(slot);
+            placed = is_empty_key(old) && claim_slot(slot, v);
+        }
+        if (!placed) {
             const unsigned long long j = atomicAdd(nextN, 1ull);
             if (j < nextCap)
                 next[j] = v;
-            else
-                atomicExch(err, 1);
         }
     }
 }
@@ -160,14 +148,8 @@ ibs_status build_wide(ibs_table *t, const ulonglong2 *dCodes, uint64_t n, uint32
     t->wide = wide::View{};
     t->wide.k = k;
     const uint64_t lines0 = std::max<uint64_t>(1, (uint64_t)((double)n / lam) + 1);
-    DevPtr<uint32_t> cnt; // per line of the level; cntCap lines
-    uint64_t cntCap = lines0;
-    DevPtr<unsigned long long> dOver; // [0] surplus keys of the level, [1] next-level fill
-    DevPtr<int> dErr;
-    IBS_CUDA(cnt.alloc(cntCap), "wide table scratch");
-    IBS_CUDA(dOver.alloc(2), "wide table scratch");
-    IBS_CUDA(dErr.alloc(1), "wide table scratch");
-    IBS_CUDA(cudaMemset(dErr.p, 0, sizeof(int)), "wide table scratch");
+    DevPtr<unsigned long long> dOver; // keys for the next level
+    IBS_CUDA(dOver.alloc(1), "wide table scratch");
     // cur: this level's input (the caller's codes, then the surplus of the
     // previous level, held by owned)
     const ulonglong2 *cur = dCodes;
@@ -181,42 +163,29 @@ ibs_status build_wide(ibs_table *t, const ulonglong2 *dCodes, uint64_t n, uint32
             return IBS_ERR_CAPACITY;
         }
         const uint64_t lines = L == 0 ? lines0 : std::max<uint64_t>(1, (nCur + 1) / 2);
-        if (lines > cntCap) {
-            cudaFree(cnt.p);
-            cnt.p = nullptr;
-            cntCap = lines;
-            IBS_CUDA(cnt.alloc(cntCap), "wide table scratch");
-        }
         ulonglong2 *slots = nullptr;
         IBS_CUDA(cudaMalloc(&slots, lines * kSlots * sizeof(ulonglong2)), "wide table alloc");
         t->wide.slots[L] = slots;
         t->wide.lines[L] = lines;
         t->wide.nLevels = L + 1;
         bytes += lines * kSlots * sizeof(ulonglong2);
-        IBS_CUDA(cudaMemset(slots, 0xff, lines * kSlots * sizeof(ulonglong2)), "wide table init");
-        IBS_CUDA(cudaMemset(cnt.p, 0, lines * sizeof(uint32_t)), "wide table counts");
-        IBS_CUDA(cudaMemset(dOver.p, 0, 2 * sizeof(unsigned long long)), "wide table counts");
-        if (nCur) {
-            k_wcount<<<grid_of(nCur, 256), 256>>>(cur, nCur, L, lines, cnt.p);
-            IBS_LAUNCHED();
-        }
-        k_wover<<<grid_of(lines, 256), 256>>>(cnt.p, lines, dOver.p);
-        IBS_LAUNCHED();
-        unsigned long long over = 0;
-        IBS_CUDA(cudaMemcpy(&over, dOver.p, sizeof over, cudaMemcpyDeviceToHost), "wide table count");
+        // about 1% of the keys find their line full at the default load; a level
+        // that leaves more is filled again with room for as many
         std::unique_ptr<DevPtr<ulonglong2>> next(new DevPtr<ulonglong2>);
-        if (over)
-            IBS_CUDA(next->alloc(over), "wide table level input");
-        if (nCur) {
-            k_wplace<<<grid_of(nCur, 256), 256>>>(cur, nCur, L, lines, cnt.p, slots, next->p, dOver.p + 1, over,
-                                                  dErr.p);
-            IBS_LAUNCHED();
-        }
-        int herr = 0;
-        IBS_CUDA(cudaMemcpy(&herr, dErr.p, sizeof herr, cudaMemcpyDeviceToHost), "wide table place");
-        if (herr) {
-            set_error("wide-key table: level input overran its count");
-            return IBS_ERR_CAPACITY;
+        unsigned long long over = 0;
+        for (uint64_t cap = nCur / 16 + 4096;;) {
+            IBS_CUDA(next->alloc(cap), "wide table level input");
+            IBS_CUDA(cudaMemset(slots, 0xff, lines * kSlots * sizeof(ulonglong2)), "wide table init");
+            IBS_CUDA(cudaMemset(dOver.p, 0, sizeof(unsigned long long)), "wide table counts");
+            if (nCur) {
+                k_wplace<<<grid_of(nCur, 256), 256>>>(cur, nCur, L, lines, slots, next->p, dOver.p, cap);
+                IBS_LAUNCHED();
+            }
+            IBS_CUDA(cudaMemcpy(&over, dOver.p, sizeof over, cudaMemcpyDeviceToHost), "wide table place");
+            if (over <= cap)
+                break;
+            cap = nCur;
+            next.reset(new DevPtr<ulonglong2>);
         }
         if (L == 0)
             stashKeys = over; // every key past level 0 stays in a later level

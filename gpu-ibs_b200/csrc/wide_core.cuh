@@ -16,8 +16,11 @@
 // The lines form up to kMaxLevels levels, each with its own line hash: level
 // 0 holds the keys at about 4 per line; the keys of lines that got more than
 // 8 go to level 1, sized at about 2 per line, and so on until none is left.
-// A probe reads its level-0 line; a hit or an empty slot ends it, a full
-// line sends it on to the next level.
+// A line's two 64-byte halves fill one after the other: a key takes the next
+// slot of its home half (a bit of its hash), then of the other half. A probe
+// therefore reads its home half; a hit or an empty last slot ends it there
+// (86% of the absent keys at 4 keys a line), a full half sends it to the other
+// one and a full line to the next level.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -39,12 +42,23 @@ struct View {
     const ulonglong2 *slots[kMaxLevels];
 };
 
-// Line of a key in one level: a 64-bit mix of both words, scaled to the
-// level's line count.
+// A 64-bit mix of both words of a key, its own in every level; scaled to the
+// level's line count it is the key's line, and its lowest bit the home half.
+IBS_HD uint64_t hash_of(uint64_t lo, uint64_t hi, uint32_t level)
+{
+    return fmix64(lo ^ fmix64(hi + 0x9e3779b97f4a7c15ull * (level + 1)));
+}
+
 IBS_HD uint64_t line_of(uint64_t lo, uint64_t hi, uint32_t level, uint64_t nLines)
 {
-    const uint64_t h = fmix64(lo ^ fmix64(hi + 0x9e3779b97f4a7c15ull * (level + 1)));
-    return mulhi64(h, nLines);
+    return mulhi64(hash_of(lo, hi, level), nLines);
+}
+
+// The slot a key's home half starts at.
+IBS_HD uint64_t home_of(uint64_t lo, uint64_t hi, uint32_t level, uint64_t nLines)
+{
+    const uint64_t h = hash_of(lo, hi, level);
+    return mulhi64(h, nLines) * kSlots + (h & 1) * (kSlots / 2);
 }
 
 // 2-bit symbols of x in reverse order.
@@ -106,61 +120,96 @@ __device__ __forceinline__ void canonical_at(const uint64_t *__restrict__ seq, c
                          __ldg(mask + mi + 1), G, k, acgt, clo, chi);
 }
 
-// Membership of one wide key, from level L0 on.
-__device__ __forceinline__ bool lookup(const View &t, uint64_t lo, uint64_t hi, uint32_t L0 = 0)
-{
-    for (uint32_t L = L0; L < t.nLevels; ++L) {
-        const ulonglong2 *p = t.slots[L] + line_of(lo, hi, L, t.lines[L]) * kSlots;
-        bool hit = false, room = false;
+// A half line's four slots.
+struct Half {
+    uint4 v[4];
+    __device__ __forceinline__ void load(const ulonglong2 *p)
+    {
+        load_sector(reinterpret_cast<const uint4 *>(p), v[0], v[1]);
+        load_sector(reinterpret_cast<const uint4 *>(p) + 2, v[2], v[3]);
+    }
+    __device__ __forceinline__ bool holds(uint64_t lo, uint64_t hi) const
+    {
+        bool hit = false;
 #pragma unroll
-        for (uint32_t s = 0; s < kSlots; ++s) {
-            const ulonglong2 v = __ldg(p + s);
-            hit |= (v.x == lo) & (v.y == hi);
-            room |= (v.x == kEmpty) & (v.y == kEmpty);
-        }
-        if (hit)
+        for (int s = 0; s < 4; ++s)
+            hit |= (v[s].x == (uint32_t)lo) & (v[s].y == (uint32_t)(lo >> 32)) & (v[s].z == (uint32_t)hi) &
+                   (v[s].w == (uint32_t)(hi >> 32));
+        return hit;
+    }
+    __device__ __forceinline__ bool full() const { return (v[3].x & v[3].y & v[3].z & v[3].w) != 0xffffffffu; }
+};
+
+// Membership of one wide key whose home half in level 0, starting at slot
+// `home`, is full without it: the line's other half, then the next levels.
+__device__ __forceinline__ bool lookup_rest(const View &t, uint64_t lo, uint64_t hi, uint64_t home)
+{
+    for (uint32_t L = 0;;) {
+        Half x;
+        x.load(t.slots[L] + (home ^ (kSlots / 2)));
+        if (x.holds(lo, hi))
             return true;
-        if (room)
+        if (!x.full() || ++L == t.nLevels)
+            return false;
+        home = home_of(lo, hi, L, t.lines[L]);
+        x.load(t.slots[L] + home);
+        if (x.holds(lo, hi))
+            return true;
+        if (!x.full())
             return false;
     }
-    return false;
 }
 
-// Membership of the warp's 32 keys (one per lane; lanes with want == false
-// take part and get false). Level 0 is read cooperatively: in each of 8
-// steps, the four 8-lane groups read four keys' lines, lane i of a group
-// slot i, so one 16-byte load per lane covers four whole 128-byte lines
-// (instead of 32 lines touched per load when every lane reads its own
-// line); each group's 8-bit ballot slices say hit and empty slot to the key's
-// lane. A key whose level-0 line is full without it goes on to level 1 alone.
-// Every lane of the warp must call it.
-__device__ __forceinline__ bool lookup_warp(const View &t, uint64_t lo, uint64_t hi, bool want, uint32_t lane)
-{
-    const uint64_t line = want ? line_of(lo, hi, 0, t.lines[0]) : 0; // line 0 exists in every table
-    const ulonglong2 *base = t.slots[0] + (lane & 7);
-    const uint32_t group = lane >> 3;
-    uint32_t hitBits = 0, roomBits = 0;
-#pragma unroll
-    for (uint32_t g = 0; g < 8; ++g) {
-        const uint32_t owner = 4 * g + group; // the key this lane's group reads in step g
-        const uint64_t l = __shfl_sync(0xffffffffu, line, owner);
-        const uint64_t klo = __shfl_sync(0xffffffffu, lo, owner);
-        const uint64_t khi = __shfl_sync(0xffffffffu, hi, owner);
-        const ulonglong2 v = __ldg(base + l * kSlots);
-        const uint32_t m = __ballot_sync(0xffffffffu, (v.x == klo) & (v.y == khi));
-        const uint32_t e = __ballot_sync(0xffffffffu, (v.x == kEmpty) & (v.y == kEmpty));
-        if ((lane >> 2) == g) { // this lane's key is 4 g + (lane & 3), read by group lane & 3
-            hitBits = (m >> (8 * (lane & 3))) & 0xffu;
-            roomBits = (e >> (8 * (lane & 3))) & 0xffu;
-        }
+// The level-0 home halves of a warp's 32 keys, one per lane, read by pairs of
+// lanes: each lane reads half of its pair's two halves, so a key's 64 bytes
+// come by one load of two lanes. (By two loads of its own lane they are two
+// requests, which fetch a line from DRAM twice when both are in flight: 17 G
+// probes/s over 2 GB.) Every lane of the warp calls both functions.
+struct PairProbe {
+    uint4 a[2], b[2];        // this lane's share of the even and the odd lane's half
+    uint64_t lo, hi, oLo, oHi; // this lane's key and its pair's
+
+    __device__ __forceinline__ void load(const View &t, uint64_t lo_, uint64_t hi_, uint64_t home, uint32_t lane)
+    {
+        lo = lo_;
+        hi = hi_;
+        oLo = __shfl_xor_sync(0xffffffffu, lo, 1);
+        oHi = __shfl_xor_sync(0xffffffffu, hi, 1);
+        const uint64_t oHome = __shfl_xor_sync(0xffffffffu, home, 1);
+        const bool odd = lane & 1;
+        const ulonglong2 *base = t.slots[0] + (odd ? 2 : 0);
+        load_sector(reinterpret_cast<const uint4 *>(base + (odd ? oHome : home)), a[0], a[1]);
+        load_sector(reinterpret_cast<const uint4 *>(base + (odd ? home : oHome)), b[0], b[1]);
     }
-    if (!want)
-        return false;
-    if (hitBits)
-        return true;
-    if (roomBits)
-        return false;
-    return lookup(t, lo, hi, 1);
+
+    static __device__ __forceinline__ bool holds(const uint4 &v, uint64_t lo, uint64_t hi)
+    {
+        return (v.x == (uint32_t)lo) & (v.y == (uint32_t)(lo >> 32)) & (v.z == (uint32_t)hi) &
+               (v.w == (uint32_t)(hi >> 32));
+    }
+    static __device__ __forceinline__ bool taken(const uint4 &v) { return (v.x & v.y & v.z & v.w) != 0xffffffffu; }
+
+    // Whether this lane's half holds its key, and whether the half is full.
+    __device__ __forceinline__ void result(uint32_t lane, bool &hit, bool &full) const
+    {
+        const bool odd = lane & 1;
+        const uint64_t aLo = odd ? oLo : lo, aHi = odd ? oHi : hi, bLo = odd ? lo : oLo, bHi = odd ? hi : oHi;
+        const uint32_t ha = __ballot_sync(0xffffffffu, holds(a[0], aLo, aHi) || holds(a[1], aLo, aHi));
+        const uint32_t hb = __ballot_sync(0xffffffffu, holds(b[0], bLo, bHi) || holds(b[1], bLo, bHi));
+        const uint32_t fa = __ballot_sync(0xffffffffu, taken(a[1])), fb = __ballot_sync(0xffffffffu, taken(b[1]));
+        const uint32_t pair = lane & ~1u;
+        hit = ((odd ? hb : ha) >> pair) & 3u;
+        full = ((odd ? fb : fa) >> (pair + 1)) & 1u; // the odd lane has the last slot
+    }
+};
+
+// Membership of one wide key.
+__device__ __forceinline__ bool lookup(const View &t, uint64_t lo, uint64_t hi)
+{
+    const uint64_t home = home_of(lo, hi, 0, t.lines[0]);
+    Half x;
+    x.load(t.slots[0] + home);
+    return x.holds(lo, hi) || (x.full() && lookup_rest(t, lo, hi, home));
 }
 #endif
 

@@ -169,3 +169,20 @@ def test_wide_cli_panel_runs_single_scans(build_case, tmp_path):
     gold = corpus.load_golden("edge_k41")
     for db in ("db", "db2"):
         assert (out / f"{db}_v_test_5000.tsv").read_bytes().decode("latin-1") == gold["tsv"]["5000"]
+
+
+@pytest.mark.parametrize("kpb", [0.3, 4.0, 7.9, 40.0])
+def test_half_lines_and_levels(kpb):
+    """Loads from nearly empty to far past the slots: home halves, other halves
+    and later levels, present and absent keys, all-T words among them."""
+    k = 64
+    rng = np.random.default_rng(int(kpb * 10))
+    lo, hi = corpus.random_codes128(rng, 30_000, k)
+    lo[:50] = np.uint64(0xFFFFFFFFFFFFFFFF)  # the last 32 bases all T: half of an empty slot
+    # T x 32 + A x 32, its own reverse complement: the other half of one
+    lo[50], hi[50] = 0, np.uint64(0xFFFFFFFFFFFFFFFF)
+    table = ib.Table.from_codes128(lo[:20_000], hi[:20_000], k, keys_per_bucket=kpb)
+    assert table.probe128(lo[:20_000], hi[:20_000]).all()
+    kept = set(zip(lo[:20_000].tolist(), hi[:20_000].tolist()))
+    want = [(a, b) in kept for a, b in zip(lo[20_000:].tolist(), hi[20_000:].tolist())]
+    assert table.probe128(lo[20_000:], hi[20_000:]).tolist() == [int(x) for x in want]
