@@ -165,6 +165,48 @@ IBS_HD void place(uint64_t D, uint32_t k, uint32_t o, uint32_t s, uint64_t g, ui
              sector_of((uint32_t)slot, (uint32_t)(slot >> 32));
 }
 
+// Offsets of the leftmost and the rightmost smallest rank key among the w (<= 8)
+// m-mers of C; R is C's reverse complement. The m-mers come as words by shifts
+// of a known amount each from C at the top of 64 bits and from R, and the
+// offsets ride in the keys' low bits.
+IBS_HD void minimizer_offsets(uint64_t C, uint64_t R, uint32_t k, uint32_t &left, uint32_t &right)
+{
+    const uint32_t m = m_of(k), w = w_of(k), hb = 2 * m - 32, restMask = (1u << hb) - 1u;
+    const uint64_t X = C << (64 - 2 * k), R1 = R >> hb;
+    uint32_t bestL = 0xffffffffu, bestR = 0xffffffffu;
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+    for (uint32_t j = 0; j < 8; ++j) {
+        if (j >= w)
+            break;
+        const uint32_t fh = (uint32_t)((X << (2 * j)) >> 32), fl = (uint32_t)X << (2 * j);
+        const uint32_t fr = hb ? fl >> (32 - hb) : 0u;
+        const uint32_t rh = (uint32_t)(R1 >> (2 * j)), rr = (uint32_t)(R >> (2 * j)) & restMask;
+        const bool rLess = rh < fh || (rh == fh && rr < fr);
+        const uint32_t key = rank_key_of(mix(rLess ? rh : fh, rLess ? rr : fr));
+        bestL = bestL < key + j ? bestL : key + j;
+        bestR = bestR < key + (7 - j) ? bestR : key + (7 - j);
+    }
+    left = bestL & 7u;
+    right = 7u - (bestR & 7u);
+}
+
+// The place of k-mer D (D2 its reverse complement) by its minimizer at offset o.
+IBS_HD void place_at(uint64_t D, uint64_t D2, uint32_t o, const TableGeom &g, uint64_t &bucket, uint64_t &slot)
+{
+    const uint32_t k = g.k, m = m_of(k);
+    const uint64_t mmask = key_mask(2 * m);
+    const uint64_t f = (D >> (2 * (k - m - o))) & mmask, r = (D2 >> (2 * o)) & mmask;
+    const bool rev = r < f;
+    const uint64_t h = line_hash(rev ? r : f, m);
+    const uint64_t own = rev ? D2 : D; // the strand that holds the minimizer itself
+    const uint32_t at = rev ? w_of(k) - 1 - o : o;
+    slot = ((uint64_t)slot_high(own, k, at) << g.fpBits) | (h & key_mask(g.fpBits));
+    bucket = line_of(h, m, g.nBuckets / kSectorsPerLine) * kSectorsPerLine +
+             sector_of((uint32_t)slot, (uint32_t)(slot >> 32));
+}
+
 // The places of canonical k-mer C: where a scan that reads C looks (by C's
 // leftmost smallest rank key), and where one that reads the other strand
 // does. They are one place but for a k-mer whose smallest key occurs at
@@ -176,36 +218,21 @@ IBS_HD void place(uint64_t D, uint32_t k, uint32_t o, uint32_t s, uint64_t g, ui
 // the code itself.
 IBS_HD uint32_t placements(uint64_t C, const TableGeom &g, uint64_t bucket[2], uint64_t slot[2])
 {
-    const uint32_t k = g.k, m = m_of(k), w = w_of(k);
-    const uint64_t R = rc_m(C, k), mmask = key_mask(2 * m);
+    const uint64_t R = rc_m(C, g.k);
     if (R < C)
         return 0;
-    uint32_t best = 0, oL = 0, oR = 0;
-    uint64_t fL = 0, rL = 0, fR = 0, rR = 0;
-    Mixed xL{0, 0}, xR{0, 0};
-    for (uint32_t j = 0; j < w; ++j) {
-        // the m-mer at offset j and its reverse complement, from C's
-        const uint64_t f = (C >> (2 * (k - m - j))) & mmask, r = (R >> (2 * j)) & mmask;
-        const Mixed x = mix_m(f < r ? f : r, m);
-        const uint32_t key = rank_key_of(x);
-        if (j == 0 || key < best) {
-            best = key;
-            oL = j;
-            fL = f;
-            rL = r;
-            xL = x;
-        }
-        if (key <= best) {
-            oR = j;
-            fR = f;
-            rR = r;
-            xR = x;
-        }
+    const uint32_t m = m_of(g.k);
+    uint32_t left, right;
+    minimizer_offsets(C, R, g.k, left, right);
+    place_at(C, R, left, g, bucket[0], slot[0]);
+    if (left == right) {
+        if (m & 1) // never its own reverse complement
+            return 1;
+        const uint64_t f = (C >> (2 * (g.k - m - left))) & key_mask(2 * m);
+        if (f != ((R >> (2 * left)) & key_mask(2 * m)))
+            return 1;
     }
-    place(C, k, oL, rL < fL, line_hash_of(xL, m), g.nBuckets, g.fpBits, bucket[0], slot[0]);
-    if (oL == oR && fL != rL)
-        return 1;
-    place(R, k, w - 1 - oR, fR < rR, line_hash_of(xR, m), g.nBuckets, g.fpBits, bucket[1], slot[1]);
+    place_at(R, C, w_of(g.k) - 1 - right, g, bucket[1], slot[1]);
     return bucket[0] == bucket[1] && slot[0] == slot[1] ? 1 : 2;
 }
 
@@ -213,11 +240,14 @@ IBS_HD uint32_t placements(uint64_t C, const TableGeom &g, uint64_t bucket[2], u
 // not canonical.
 IBS_HD bool locate(uint64_t C, const TableGeom &g, uint64_t &bucket, uint64_t &slot)
 {
-    uint64_t b[2] = {0, 0}, s[2] = {0, 0};
-    const bool has = placements(C, g, b, s) != 0;
-    bucket = b[0];
-    slot = s[0];
-    return has;
+    const uint64_t R = rc_m(C, g.k);
+    bucket = slot = 0;
+    if (R < C)
+        return false;
+    uint32_t left, right;
+    minimizer_offsets(C, R, g.k, left, right);
+    place_at(C, R, left, g, bucket, slot);
+    return true;
 }
 
 } // namespace mz
