@@ -279,9 +279,9 @@ struct ScanPlan {
 
 // Positions per span for a reference (or a group of its windows) of `bases`:
 // the tuned length, or less where that would leave the GPU's warps without a
-// span. 1 Mbp in spans of 2048 is 490 warps on 32 of 148 SMs (51 us), in spans
-// of 256 3900 warps.
-uint32_t span_length(uint64_t bases, uint32_t tuned);
+// span (1 Mbp in spans of 2048 is 490 warps on 32 of 148 SMs, 51 us; in spans
+// of 128, 7800 warps), and cutting full windows evenly.
+uint32_t span_length(uint64_t bases, uint32_t tuned, uint32_t W, uint32_t k);
 
 // Build the plan's host arrays for contigs `lens` starting at packed
 // offsets `baseOff`.

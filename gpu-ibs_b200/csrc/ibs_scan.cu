@@ -29,14 +29,14 @@ namespace ibs {
 constexpr uint32_t FULL = 0xffffffffu;
 
 static std::mutex g_tuneMu;
-// Defaults: the autotuner's best point on the B200 (gpu-ibs_b200/tuning/b200.json,
-// plain 2 Gbp x 2.19e9 k-mers): minimizer table at 1.5 keys per 32-byte
-// sector, spans of 2048 positions, 2 blocks in flight, 512 threads, 16 CTAs
-// per SM.
-// Joint-table scans (the autotuner's best point on the 16-sample panel at
-// half size): spans of 8192 positions, 4 CTAs of 256 threads per SM, 2
-// blocks in flight, 3 keys per 5-slot bucket.
-static ibs_tuning g_tune = {2048, 2, 512, 16, 1.5, FMT_MZ8, 0, 8192, 4, 3.0, 2, {0, 0, 0}};
+// Defaults: minimizer table at 1.5 keys per 32-byte sector, 16 CTAs of 512
+// threads per SM with 2 blocks in flight for hash buckets (the autotuner's
+// sweep, gpu-ibs_b200/tuning/b200.json), spans of up to 8192 positions (1 Gbp at
+// k = 25 against spans of 2048 / 4096 / 8192: 6.57 / 6.43 / 6.34 ms).
+// Joint-table scans: spans of up to 4096 positions (200 Mbp against 16 samples
+// at k = 31 with 1024 / 4096 / 8192: 2.24 / 2.18 / 2.24 ms), 4 CTAs of 256 threads
+// per SM, 2 blocks in flight, 3 keys per 5-slot bucket.
+static ibs_tuning g_tune = {8192, 2, 512, 16, 1.5, FMT_MZ8, 0, 4096, 4, 3.0, 2, {0, 0, 0}};
 
 const ibs_tuning &tuning() { return g_tune; }
 
@@ -246,14 +246,20 @@ void ScanPlan::release()
     span0.clear();
 }
 
-// Below 128 positions a span has less than one block of the minimizer-line
-// scan; 24 warps a SM are what the scan kernels keep resident.
-uint32_t span_length(uint64_t bases, uint32_t tuned)
+// 24 warps a SM are what the scan kernels keep resident; with four spans each
+// they even out (16 Mbp of wide keys: 377 us with two, 345 with four), but short
+// spans have more to sum up (1 Mbp: 50 us with one span of 256 a warp, 57 with two
+// of 128). Below 128 positions a span has less than one block of the
+// minimizer-line scan. Then the length that cuts a full window into equal spans
+// of whole blocks: 50 kbp in spans of 4096 would leave one of 824.
+uint32_t span_length(uint64_t bases, uint32_t tuned, uint32_t W, uint32_t k)
 {
     const uint64_t warps = (uint64_t)sm_count() * 24;
-    while (tuned >= 256 && tuned % 256 == 0 && bases / tuned < warps)
+    while (tuned >= 256 && tuned % 256 == 0 && bases / tuned < warps * (tuned > 512 ? 4 : 1))
         tuned /= 2;
-    return tuned;
+    const uint32_t blocks = (W - k + 1 + 127) / 128, want = tuned / 128;
+    const uint32_t n = (blocks + want - 1) / want; // spans a window
+    return n <= 1 ? tuned : (blocks + n - 1) / n * 128;
 }
 
 void plan_windows(ScanPlan &p, const std::vector<uint64_t> &lens,
@@ -711,7 +717,7 @@ static ibs_status ensure_plan(ibs_reference *r, uint32_t W, uint32_t k)
     uint64_t bases = 0;
     for (uint64_t l : r->lens)
         bases += l;
-    const uint32_t spanLen = span_length(bases, tuning().span_len);
+    const uint32_t spanLen = span_length(bases, tuning().span_len, W, k);
     if (p.dWin && p.W == W && p.k == k && p.spanLen == spanLen)
         return IBS_OK;
     IBS_CUDA(cudaStreamSynchronize(r->stream), "plan sync");
@@ -969,7 +975,7 @@ extern "C" ibs_status ibs_scan_packed(ibs_table *t, const uint64_t *seq2bit,
     std::vector<uint64_t> lv(lens, lens + n);
     ScanPlan &p = ws.plan;
     // the windows go in groups, the first a 128th of the reference
-    plan_windows(p, lv, off, W, k, span_length((seqWords - 1) * 32 / 8, tuning().span_len));
+    plan_windows(p, lv, off, W, k, span_length((seqWords - 1) * 32 / 8, tuning().span_len, W, k));
     if (p.nSpans > ws.spansCap || !p.dSpans) {
         cudaFree(p.dSpans);
         p.dSpans = nullptr;
