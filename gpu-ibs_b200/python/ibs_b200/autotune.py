@@ -84,7 +84,7 @@ def sweep(scale: float = 0.25, reps: int = 3, quick: bool = False) -> dict:
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     base = get_tuning()
     layouts = [(1, 3.0), (4, 2.0)] if quick else [(1, 3.0), (1, 4.0), (4, 1.5), (4, 2.0), (4, 3.0)]
-    shapes = list(itertools.product([4096] if quick else [1024, 2048, 4096],
+    shapes = list(itertools.product([4096] if quick else [1024, 2048, 4096, 8192],
                                     [2, 4] if quick else [1, 2, 4],
                                     [256, 512],
                                     [8, 16]))
