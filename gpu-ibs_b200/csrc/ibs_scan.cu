@@ -33,10 +33,10 @@ static std::mutex g_tuneMu;
 // threads per SM with 2 blocks in flight for hash buckets (the autotuner's
 // sweep, gpu-ibs_b200/tuning/b200.json), spans of up to 8192 positions (1 Gbp at
 // k = 25 against spans of 2048 / 4096 / 8192: 6.57 / 6.43 / 6.34 ms).
-// Joint-table scans: spans of up to 4096 positions (200 Mbp against 16 samples
-// at k = 31 with 1024 / 4096 / 8192: 2.24 / 2.18 / 2.24 ms), 4 CTAs of 256 threads
-// per SM, 2 blocks in flight, 3 keys per 5-slot bucket.
-static ibs_tuning g_tune = {8192, 2, 512, 16, 1.5, FMT_MZ8, 0, 4096, 4, 3.0, 2, {0, 0, 0}};
+// Joint-table scans (the autotuner's best point on the 16-sample panel at
+// half size): spans of up to 8192 positions, 4 CTAs of 256 threads per SM, 2
+// blocks in flight, 3 keys per 5-slot bucket.
+static ibs_tuning g_tune = {8192, 2, 512, 16, 1.5, FMT_MZ8, 0, 8192, 4, 3.0, 2, {0, 0, 0}};
 
 const ibs_tuning &tuning() { return g_tune; }
 
