@@ -155,7 +155,7 @@ __device__ __forceinline__ bool stash_insert(uint64_t *stash, uint64_t stashBuck
 // (k_fill): the bucket is read and the slot claimed by a compare-and-swap on
 // the same line, so a key costs one random line. (Counting the keys of every
 // bucket first and placing them in a second pass touched three: 14 ms against
-// 6 for 220M keys.) Keys that find no slot go to a list, and a second, small
+// 7 for 220M keys.) Keys that find no slot go to a list, and a second, small
 // pass (k_spill) settles those.
 
 // Claims one of 32-bit slots [0, last) of a B8x32 bucket for fp, the first free
