@@ -6,6 +6,7 @@
 
 #include <atomic>
 #include <cstdint>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -212,6 +213,7 @@ struct ibs_table {
     double buildSeconds = 0;
     uint64_t deviceBytes = 0;
     ibs::wide::View wide{}; // the levels of a wide-key table (geom.format == FMT_WIDE)
+    std::mutex countMu;     // held by a membership count: its total lies behind the buckets
     ibs::TableView view() const { return ibs::TableView{geom, buckets, stash}; }
 };
 

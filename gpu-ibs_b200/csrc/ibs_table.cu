@@ -1049,6 +1049,7 @@ static ibs_status count_present_device(ibs_table *t, const uint64_t *dCodes, uin
     *count = 0;
     if (!n)
         return IBS_OK;
+    std::lock_guard<std::mutex> lock(t->countMu);
     unsigned long long *dCount = reinterpret_cast<unsigned long long *>(t->buckets + 2 * t->geom.nBuckets);
     IBS_CUDA(cudaMemsetAsync(dCount, 0, sizeof *dCount, 0), "count init");
     const int grid = grid_for(n, 256);
