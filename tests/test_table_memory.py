@@ -1,0 +1,41 @@
+"""The device memory that tables of the default layouts take: what callers who
+keep many tables, or serve them under a budget, have planned."""
+import numpy as np
+import pytest
+
+import ibs_b200 as ib
+
+
+@pytest.mark.parametrize("k,log2_lines", [(20, 13), (23, 19), (25, 23), (27, 27), (28, 20), (31, 26)])
+def test_default_layout_by_size(k, log2_lines):
+    """Minimizer lines (1.5 keys a 32-byte sector of four a line) from 2^log2_lines
+    lines on, hash sectors of 4 keys below: the smallest line count that slot
+    values allow is half of that, and such tables are not oversized for it."""
+    first = 6 << log2_lines
+    lines = ib.table_bytes_for(first, k)
+    assert lines >= (128 << log2_lines)
+    for n in (first - 6, first * 3 // 4, first // 2 + 6):
+        hashed = ib.table_bytes_for(n, k, force_format=5)
+        assert ib.table_bytes_for(n, k) == hashed < 0.55 * lines
+
+
+@pytest.mark.gpu
+def test_tables_of_hash_sectors_fit_a_small_budget():
+    """Four samples whose hash sectors a budget holds all at once; on minimizer
+    lines (which k = 20 allows from 2^12 lines) one of them would not fit."""
+    k, W, n = 20, 1000, 30_000
+    rng = np.random.default_rng(3)
+    text = np.frombuffer(b"ACGT", np.uint8)[rng.integers(0, 4, 50_000)].tobytes()
+    ref = ib.Reference(*ib.pack_ascii([text]))
+    one = ib.table_bytes_for(n, k, force_format=5)
+    srv = ib.Server(ref, W, k, memory_budget=int(4.4 * one))
+    codes = [np.unique(rng.integers(0, 1 << 38, n).astype(np.uint64)) for _ in range(4)]
+    for i, c in enumerate(codes):
+        assert srv.add_codes(c, len(c), on_device=False) == i
+    st = srv.stats()
+    assert st["resident_tables"] == 4 and st["resident_bytes"] <= 4.4 * one
+    srv.close()
+    t = ib.Table.from_codes(codes[0], len(codes[0]), k, on_device=False)
+    assert t.info().format == 1
+    lined = ib.Table.from_codes(codes[0], len(codes[0]), k, on_device=False, force_format=4)
+    assert lined.info().device_bytes > 2 * one
