@@ -21,7 +21,7 @@ constexpr uint64_t kStashProbe = 64;
 // sectors' 3)
 constexpr double kPmKeysPerSector = 1.5;
 constexpr double kPm6KeysPerSector = 1.2; // the same share of a sector's four slots
-constexpr uint64_t kBuildChunk = 1ull << 27; // keys per build step (1 GiB of scratch each way)
+constexpr uint64_t kBuildChunk = 1ull << 27; // places of keys per build step (1 GiB of scratch each way)
 
 // Slot of fingerprint (or slot value) fp among sector w's first count slots,
 // or -1. wide: four 40-bit slot values (PM6).
@@ -489,56 +489,61 @@ extern "C" ibs_status ibs_panel_table_create(uint32_t k, uint64_t expected_keys,
     const uint64_t pmLines = (uint64_t)((double)expected_keys / lamPm / mz::kSectorsPerLine) + 1;
     if (fmt == 0 && k >= 16 && k <= 27 && pmLines >= pmMinLines && pmLines < (1ull << 31))
         fmt = FMT_PANEL_MZ; // the default where its minimum size does not oversize the table
+    // hash sectors at their load, and the stash of minimizer lines at theirs
+    const double lamHash = (opts && opts->keys_per_bucket > 0) ? opts->keys_per_bucket : tuning().panel_keys_per_bucket;
+    uint64_t hashSectors = std::max((uint64_t)((double)expected_keys / lamHash) + 1,
+                                    (uint64_t)(g.bits > 32 ? 1ull << (g.bits - 32) : 1));
+    if (g.bits < 64)
+        hashSectors = std::min<uint64_t>(hashSectors, 1ull << g.bits);
+    // minimizer lines: the keys of one minimizer crowd its line, so far more
+    // than a Poisson share of them overflows (about 2% at 1.5 keys per
+    // sector, 10% at 3); sized here for twice that, the stash grows if needed
+    auto lineStash = [&](double lam, double most) {
+        const double over = (double)expected_keys * std::min(0.5, 0.04 * lam / most * lam / most + 0.01);
+        return next_pow2(std::max<uint64_t>(1u << 12, (uint64_t)(over * 0.75) + 1));
+    };
     // k = 28 .. 31, at the default load: minimizer lines of 40-bit slots where
     // their minimum size does not oversize the table, it stays within one
-    // bucket-range pass and there is room for it. (Hash sectors cost a random
-    // line a position: 200 Mbp against 16 samples 4.5 ms, on lines 2.2 ms. But
-    // they take half the memory, and past 48 GiB random lines get slow. A caller
-    // who gives a load has planned for the hash sectors'.)
+    // bucket-range pass, and it never takes more memory than the hash sectors
+    // would, also while the stash doubles (old and new together are three times
+    // it). A line takes 26.7 bytes a key and a hash sector 10.7, but hash
+    // sectors of 32-bit fingerprints are at least 2^(2k-32): 34 GB at k = 31,
+    // where lines are the smaller layout up to 1.0e9 keys. (Scans: 200 Mbp
+    // against 16 samples 4.5 ms on hash sectors, 2.2 ms on lines. A caller who
+    // gives a load gets hash sectors.)
     const uint64_t pm6Lines = (uint64_t)((double)expected_keys / kPm6KeysPerSector / mz::kSectorsPerLine) + 1;
     if (fmt == 0 && k >= 28 && k <= 31 && !(opts && opts->keys_per_bucket > 0) && pm6Lines >= 1ull << (2 * k - 37) &&
-        pm6Lines * 128 <= 48ull << 30) {
-        size_t freeBytes = 0, totalBytes = 0;
-        IBS_CUDA(cudaMemGetInfo(&freeBytes, &totalBytes), "cudaMemGetInfo");
-        if (pm6Lines * 128 + pm6Lines * 16 <= freeBytes)
-            fmt = FMT_PANEL_MZ6;
-    }
+        pm6Lines * 128 <= 48ull << 30 &&
+        pm6Lines * 128 + 3 * lineStash(kPm6KeysPerSector, kPm6KeysPerSector) * 32 <= hashSectors * 32)
+        fmt = FMT_PANEL_MZ6;
     if (fmt == 0)
         fmt = FMT_PANEL;
     g.format = fmt;
     uint64_t nb;
-    double lam;
     if (fmt == FMT_PANEL_MZ) {
-        lam = lamPm;
         const uint64_t nLines = std::min<uint64_t>(std::max(pmLines, pmMinLines), (1ull << 31) - 1);
         nb = nLines * mz::kSectorsPerLine;
         g.nBuckets = nb;
         g.fpBits = 2 * mz::m_of(k) - (uint32_t)(63 - __builtin_clzll(nLines));
     } else if (fmt == FMT_PANEL_MZ6) {
-        lam = kPm6KeysPerSector;
         nb = pm6Lines * mz::kSectorsPerLine;
         g.nBuckets = nb;
         g.fpBits = 2 * mz::m_of(k) - (uint32_t)(63 - __builtin_clzll(pm6Lines));
     } else {
-        lam = (opts && opts->keys_per_bucket > 0) ? opts->keys_per_bucket : tuning().panel_keys_per_bucket;
-        nb = (uint64_t)((double)expected_keys / lam) + 1;
-        const uint64_t minN = g.bits > 32 ? (1ull << (g.bits - 32)) : 1;
-        nb = std::max(nb, minN);
-        if (g.bits < 64)
-            nb = std::min<uint64_t>(nb, 1ull << g.bits);
+        nb = hashSectors;
         g.nBuckets = nb;
         g.fpBits = (uint32_t)std::max<int>(1, (int)g.bits - (int)(63 - __builtin_clzll(nb)));
     }
-    // keys per bucket are ~Poisson(expected / nBuckets); the stash holds the
-    // expected overflow at <= 2/3 load (it grows during the build if needed)
-    // minimizer lines: the keys of one minimizer crowd its line, so far more
-    // than a Poisson share of them overflows (about 2% at 1.5 keys per
-    // sector, 10% at 3); sized here for twice that, the stash grows if needed
-    const double most = fmt == FMT_PANEL_MZ6 ? kPm6KeysPerSector : kPmKeysPerSector;
-    const double over = is_joint_mz(fmt)
-                            ? (double)expected_keys * std::min(0.5, 0.04 * lam / most * lam / most + 0.01)
-                            : (double)expected_keys * overflow_fraction((double)expected_keys / (double)nb);
-    p->stashBuckets = next_pow2(std::max<uint64_t>(1u << 12, (uint64_t)(over * 0.75) + 1));
+    // hash sectors: keys per bucket are ~Poisson(expected / nBuckets); the stash
+    // holds the expected overflow at <= 2/3 load (it grows during the build if
+    // needed)
+    if (is_joint_mz(fmt)) {
+        p->stashBuckets = fmt == FMT_PANEL_MZ6 ? lineStash(kPm6KeysPerSector, kPm6KeysPerSector)
+                                               : lineStash(lamPm, kPmKeysPerSector);
+    } else {
+        const double over = (double)expected_keys * overflow_fraction((double)expected_keys / (double)nb);
+        p->stashBuckets = next_pow2(std::max<uint64_t>(1u << 12, (uint64_t)(over * 0.75) + 1));
+    }
     g.stashBuckets = p->stashBuckets;
     IBS_CUDA(cudaMalloc(&p->buckets, nb * 32), "panel table alloc");
     IBS_CUDA(cudaMemset(p->buckets, 0, nb * 32), "panel table init");
@@ -607,9 +612,9 @@ static ibs_status panel_add_device_codes(ibs_panel_table *p, const uint64_t *dCo
         p->graph = nullptr;
     }
     // keys go in chunks, so the build's scratch stays small next to the table
-    const uint64_t chunk = std::max<uint64_t>(1, std::min<uint64_t>(n, kBuildChunk));
     uint64_t *pending = nullptr, *failed = nullptr;
     const uint64_t places = is_joint_mz(p->geom.format) ? 2 : 1; // most places a key has
+    const uint64_t chunk = std::max<uint64_t>(1, std::min<uint64_t>(n, kBuildChunk / places));
     IBS_CUDA(cudaMalloc(&pending, chunk * places * 8), "panel pending alloc");
     std::unique_ptr<uint64_t, cudaError_t (*)(void *)> g1(pending, cudaFree);
     IBS_CUDA(cudaMalloc(&failed, chunk * places * 8), "panel pending alloc");

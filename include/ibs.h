@@ -267,9 +267,9 @@ ibs_status ibs_scan_panel(ibs_table *const *tables, uint32_t n_tables, ibs_refer
  * the stash; default load 1.5 keys per sector); 0 = 7 where it applies and its
  * minimum size does not oversize the table, for 28 <= k <= 31 the same with
  * 40-bit slots (reported as format 9; four slots a sector, at least 2^(2k-37)
- * lines, at the default load, up to 48 GiB and where the device has room), else
- * 3. opts->keys_per_bucket: keys
- * per sector (0 = the tuned panel_keys_per_bucket for 3, 1.5 for 7). Samples are added one at a
+ * lines, at the default load, up to 48 GiB and where 3 would take no less
+ * memory), else 3. opts->keys_per_bucket: keys per sector (0 = the tuned
+ * panel_keys_per_bucket for 3, 1.5 for 7). Samples are added one at a
  * time (sample i = the i-th call); rows are sample-major:
  * rows[i * n_windows + w]. The scan is a persistent kernel over a work queue
  * of (window, position-range) spans; ibs_panel_table_scan_async captures it

@@ -39,3 +39,21 @@ def test_tables_of_hash_sectors_fit_a_small_budget():
     assert t.info().format == 1
     lined = ib.Table.from_codes(codes[0], len(codes[0]), k, on_device=False, force_format=4)
     assert lined.info().device_bytes > 2 * one
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("k,few,many", [(28, 3_000_000, 30_000_000), (29, 11_000_000, 90_000_000)])
+def test_joint_lines_take_no_more_than_hash_sectors(k, few, many):
+    """Joint tables of k = 28 .. 31: minimizer lines (format 9) while they fit in
+    the 2^(2k - 32) hash sectors that the keys would take at least, with room
+    for the stash to double; hash sectors beyond that, and for a given load."""
+    sectors = 32 << (2 * k - 32)
+    for n, fmt in ((few, 9), (many, 3)):
+        pt = ib.PanelTable(k, n)
+        info = pt.info()[0]
+        assert info.format == fmt
+        assert info.device_bytes + 2 * info.stash_buckets * 32 <= 1.05 * sectors
+        pt.close()
+    pt = ib.PanelTable(k, few, keys_per_bucket=3.0)
+    assert pt.info()[0].format == 3
+    pt.close()
