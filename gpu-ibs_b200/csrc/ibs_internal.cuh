@@ -228,19 +228,22 @@ struct WinDesc {
 
 #if defined(__CUDACC__)
 namespace dev {
-// A window's row from its n span summaries, by one warp: each lane combines a
-// run of consecutive summaries, and a shuffle tree the 32 runs in order. (One
-// thread a window took 20 us for the 25 spans of a 50 kbp window, each load
-// waiting for the one before; small references have 200 shorter spans.)
-__device__ __forceinline__ void finish_window(const WinDesc &w, const SegStats *__restrict__ spans, uint32_t n, int k,
-                                              uint32_t lane, ibs_window *__restrict__ out)
+// A window's row from its n span summaries, by a group of 2^log2 lanes (lane
+// `at` of the group calls it, every lane of the warp does; n = 0 and no row for
+// a group without a window): each lane combines a run of consecutive summaries,
+// and a shuffle tree the group's runs in order. The group is as wide as a
+// window has spans (finish_lanes): one thread a window took 20 us for the 25
+// spans of a 50 kbp window, each load waiting for the one before, and a warp
+// for each of the one-span windows of a small W cost more than the scan itself
+// (8 samples at W = 64, k = 25: 3.2 ms against 1.4).
+__device__ __forceinline__ void finish_window(const WinDesc *w, const SegStats *__restrict__ spans, uint32_t n, int k,
+                                              uint32_t at, uint32_t log2, ibs_window *__restrict__ out)
 {
-    const uint32_t run = (n + 31) / 32, a = min(lane * run, n), b = min(a + run, n);
+    const uint32_t run = (n + (1u << log2) - 1) >> log2, a = min(at * run, n), b = min(a + run, n);
     SegStats acc = seg_empty();
     for (uint32_t s = a; s < b; ++s)
         acc = seg_combine(acc, spans[s], k);
-#pragma unroll
-    for (uint32_t off = 1; off < 32; off <<= 1) {
+    for (uint32_t off = 1; off < 1u << log2; off <<= 1) {
         SegStats o;
         o.total = __shfl_down_sync(0xffffffffu, acc.total, off);
         o.obs = __shfl_down_sync(0xffffffffu, acc.obs, off);
@@ -249,14 +252,14 @@ __device__ __forceinline__ void finish_window(const WinDesc &w, const SegStats *
         o.gaps = __shfl_down_sync(0xffffffffu, acc.gaps, off);
         o.dist = __shfl_down_sync(0xffffffffu, acc.dist, off);
         o.pad = 0;
-        acc = seg_combine(acc, o, k); // right for lanes that are multiples of 2 off
+        acc = seg_combine(acc, o, k); // right for lanes that are multiples of 2 off in their group
     }
-    if (lane == 0) {
+    if (at == 0 && out) {
         WindowRow row;
         seg_finish(acc, k, row);
         ibs_window o;
-        o.start = w.start;
-        o.end = w.end;
+        o.start = w->start;
+        o.end = w->end;
         o.total_kmers = row.total_kmers;
         o.observed_kmers = row.observed_kmers;
         o.variations = row.variations;
@@ -271,6 +274,7 @@ __device__ __forceinline__ void finish_window(const WinDesc &w, const SegStats *
 struct ScanPlan {
     uint32_t W = 0, k = 0, spanLen = 0;
     uint64_t nWin = 0, nSpans = 0;
+    uint32_t maxSpans = 0;        // of one window
     std::vector<WinDesc> win;     // host copy
     std::vector<uint32_t> span0;  // host copy, nWin + 1
     WinDesc *dWin = nullptr;
@@ -278,6 +282,12 @@ struct ScanPlan {
     SegStats *dSpans = nullptr;   // scratch: one summary per span
     void release();
 };
+
+// log2 of the lanes that finish each of `windows` windows of the plan: as many
+// as a window has spans, up to a warp. As many as the largest one has while
+// that leaves lanes of the GPU idle (a few long contigs among many short ones),
+// as many as there are on average otherwise.
+uint32_t finish_lanes(const ScanPlan &p, uint64_t windows);
 
 // Positions per span for a reference (or a group of its windows) of `bases`:
 // the tuned length, or less where that would leave the GPU's warps without a

@@ -385,15 +385,17 @@ __global__ void __launch_bounds__(256, 3) k_panel_spans_mz(const __grid_constant
 __global__ void __launch_bounds__(256) k_panel_finalize(const WinDesc *__restrict__ win,
                                                         const uint32_t *__restrict__ span0, uint64_t nWin,
                                                         uint64_t nSpans, uint32_t nSamples,
-                                                        const SegStats *__restrict__ spans, int k,
+                                                        const SegStats *__restrict__ spans, int k, uint32_t log2,
                                                         ibs_window *__restrict__ rows)
 {
-    const uint32_t lane = threadIdx.x & 31;
-    const uint64_t total = nWin * nSamples, nWarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t x = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; x < total; x += nWarps) {
-        const uint64_t smp = x / nWin, w = x - smp * nWin;
-        const uint32_t s0 = span0[w];
-        dev::finish_window(win[w], spans + smp * nSpans + s0, span0[w + 1] - s0, k, lane, rows + x);
+    const uint32_t lane = threadIdx.x & 31, group = lane >> log2, at = lane & ((1u << log2) - 1);
+    const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5, total = nWin * nSamples;
+    const uint64_t step = (((uint64_t)gridDim.x * blockDim.x) >> 5) << (5 - log2);
+    for (uint64_t x0 = warp << (5 - log2); x0 < total; x0 += step) {
+        const uint64_t x = x0 + group, smp = x / nWin, w = x - smp * nWin;
+        const bool have = x < total;
+        const uint32_t s0 = have ? span0[w] : 0, n = have ? span0[w + 1] - s0 : 0;
+        dev::finish_window(win + w, spans + smp * nSpans + s0, n, k, at, log2, have ? rows + x : nullptr);
     }
 }
 
@@ -845,8 +847,9 @@ static ibs_status panel_enqueue(ibs_panel_table *p, const ibs_reference *ref, ib
             return s;
     }
     if (pl.nWin && p->nSamples) {
-        k_panel_finalize<<<grid_for(pl.nWin * p->nSamples * 32), 256, 0, st>>>(
-            pl.dWin, pl.dSpan0, pl.nWin, pl.nSpans, p->nSamples, p->dSpans, (int)p->geom.k, rowsDev);
+        const uint32_t log2 = finish_lanes(pl, pl.nWin * p->nSamples);
+        k_panel_finalize<<<grid_for(pl.nWin * p->nSamples << log2), 256, 0, st>>>(
+            pl.dWin, pl.dSpan0, pl.nWin, pl.nSpans, p->nSamples, p->dSpans, (int)p->geom.k, log2, rowsDev);
         IBS_LAUNCHED();
     }
     IBS_CUDA(cudaGetLastError(), "panel scan launch");

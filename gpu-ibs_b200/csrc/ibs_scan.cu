@@ -214,13 +214,16 @@ __global__ void __launch_bounds__(kMzThreads, 3) k_scan_spans_mz(const __grid_co
 
 __global__ void __launch_bounds__(256) k_finalize(const WinDesc *__restrict__ win, const uint32_t *__restrict__ span0,
                                                   uint64_t nWin, const SegStats *__restrict__ spans, int k,
-                                                  ibs_window *__restrict__ rows)
+                                                  uint32_t log2, ibs_window *__restrict__ rows)
 {
-    const uint32_t lane = threadIdx.x & 31;
-    const uint64_t nWarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t w = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; w < nWin; w += nWarps) {
-        const uint32_t s0 = span0[w];
-        dev::finish_window(win[w], spans + s0, span0[w + 1] - s0, k, lane, rows + w);
+    const uint32_t lane = threadIdx.x & 31, group = lane >> log2, at = lane & ((1u << log2) - 1);
+    const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+    const uint64_t step = (((uint64_t)gridDim.x * blockDim.x) >> 5) << (5 - log2);
+    for (uint64_t w0 = warp << (5 - log2); w0 < nWin; w0 += step) {
+        const uint64_t w = w0 + group;
+        const bool have = w < nWin;
+        const uint32_t s0 = have ? span0[w] : 0, n = have ? span0[w + 1] - s0 : 0;
+        dev::finish_window(win + w, spans + s0, n, k, at, log2, have ? rows + w : nullptr);
     }
 }
 
@@ -262,6 +265,15 @@ uint32_t span_length(uint64_t bases, uint32_t tuned, uint32_t W, uint32_t k)
     return n <= 1 ? tuned : (blocks + n - 1) / n * 128;
 }
 
+uint32_t finish_lanes(const ScanPlan &p, uint64_t windows)
+{
+    const uint64_t idle = (uint64_t)sm_count() * 2048, each = p.nWin ? (p.nSpans + p.nWin - 1) / p.nWin : 1;
+    uint32_t log2 = 0;
+    while (log2 < 5 && 1u << log2 < p.maxSpans && (1u << log2 < each || windows << (log2 + 1) <= idle))
+        ++log2;
+    return log2;
+}
+
 void plan_windows(ScanPlan &p, const std::vector<uint64_t> &lens,
                   const std::vector<uint64_t> &baseOff, uint32_t W, uint32_t k, uint32_t spanLen)
 {
@@ -270,6 +282,7 @@ void plan_windows(ScanPlan &p, const std::vector<uint64_t> &lens,
     p.W = W;
     p.k = k;
     p.spanLen = spanLen;
+    p.maxSpans = 0;
     uint64_t spans = 0;
     const uint64_t step = (uint64_t)W - k;
     for (size_t c = 0; c < lens.size(); ++c) {
@@ -285,7 +298,9 @@ void plan_windows(ScanPlan &p, const std::vector<uint64_t> &lens,
             d.pad = 0;
             p.win.push_back(d);
             p.span0.push_back((uint32_t)spans);
-            spans += (d.nPos + spanLen - 1) / spanLen;
+            const uint32_t n = (d.nPos + spanLen - 1) / spanLen;
+            p.maxSpans = std::max(p.maxSpans, n);
+            spans += n;
         }
     }
     p.span0.push_back((uint32_t)spans);
@@ -377,9 +392,10 @@ static ibs_status launch_finalize_with(const ScanPlan &p, uint32_t k, const SegS
     if (!p.nWin)
         return IBS_OK;
     const int threads = 256;
-    const uint64_t want = (p.nWin * 32 + threads - 1) / threads;
+    const uint32_t log2 = finish_lanes(p, p.nWin);
+    const uint64_t want = ((p.nWin << log2) + threads - 1) / threads;
     const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>(want, (uint64_t)sm_count() * 8));
-    k_finalize<<<grid, threads, 0, st>>>(p.dWin, p.dSpan0, p.nWin, dSpans, (int)k, dRows);
+    k_finalize<<<grid, threads, 0, st>>>(p.dWin, p.dSpan0, p.nWin, dSpans, (int)k, log2, dRows);
     IBS_LAUNCHED();
     IBS_CUDA(cudaGetLastError(), "finalize kernel launch");
     return IBS_OK;
