@@ -227,19 +227,6 @@ __global__ void k_stash_move(const ulonglong2 *old, uint64_t oldEntries, unsigne
 // one range.
 enum : int { kScan = 0, kMaskPass = 1, kStats = 2 };
 
-__device__ __forceinline__ uint32_t window_of(const uint32_t *__restrict__ span0, uint32_t nWin, uint64_t s)
-{
-    uint32_t lo = 0, hi = nWin - 1;
-    while (lo < hi) {
-        const uint32_t mid = (lo + hi + 1) >> 1;
-        if (__ldg(span0 + mid) <= s)
-            lo = mid;
-        else
-            hi = mid - 1;
-    }
-    return lo;
-}
-
 // The hash-sector tables (P5x48), and the statistics pass of either layout.
 template <int NB, int MODE>
 __global__ void __launch_bounds__(256) k_panel_spans(View t, const uint64_t *__restrict__ seq,
@@ -263,7 +250,7 @@ __global__ void __launch_bounds__(256) k_panel_spans(View t, const uint64_t *__r
         s = __shfl_sync(dev::FULL_MASK, s, 0);
         if (s >= nSpans)
             break;
-        const uint32_t lo = window_of(span0, nWin, s);
+        const uint32_t lo = dev::window_of_span(span0, nWin, s, lane);
         const uint64_t base = win[lo].base;
         const uint32_t nPos = win[lo].nPos;
         const uint32_t p0 = (uint32_t)(s - __ldg(span0 + lo)) * spanLen;
@@ -352,7 +339,7 @@ __global__ void __launch_bounds__(256, 3) k_panel_spans_mz(const __grid_constant
         s = __shfl_sync(dev::FULL_MASK, s, 0);
         if (s >= nSpans)
             break;
-        const uint32_t w = window_of(span0, nWin, s);
+        const uint32_t w = dev::window_of_span(span0, nWin, s, lane);
         const uint64_t base = win[w].base;
         const uint32_t nPos = win[w].nPos;
         const uint32_t p0 = (uint32_t)(s - __ldg(span0 + w)) * spanLen;

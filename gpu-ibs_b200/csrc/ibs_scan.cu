@@ -52,20 +52,6 @@ __device__ __forceinline__ void fold_blocks(dev::LaneFold<> &fold, const uint32_
         fold.push(V[b], H[b], lane, k);
 }
 
-__device__ __forceinline__ uint32_t window_of_span(const uint32_t *__restrict__ span0,
-                                                   uint32_t nWin, uint64_t s)
-{
-    uint32_t lo = 0, hi = nWin - 1;
-    while (lo < hi) {
-        const uint32_t mid = (lo + hi + 1) >> 1;
-        if (__ldg(span0 + mid) <= s)
-            lo = mid;
-        else
-            hi = mid - 1;
-    }
-    return lo;
-}
-
 template <uint32_t FMT, int NB>
 __global__ void __launch_bounds__(512) k_scan_spans(TableView t, const uint64_t *__restrict__ seq,
                                                     const uint64_t *__restrict__ mask,
@@ -81,7 +67,7 @@ __global__ void __launch_bounds__(512) k_scan_spans(TableView t, const uint64_t 
     const uint64_t kmask = key_mask(2 * k);
     const uint64_t kbits = (1ull << k) - 1; // k <= 32
     for (uint64_t s = s0 + warp; s < s1; s += nWarps) {
-        const uint32_t w = window_of_span(span0, nWin, s);
+        const uint32_t w = dev::window_of_span(span0, nWin, s, lane);
         const uint64_t base = win[w].base;
         const uint32_t nPos = win[w].nPos;
         const uint32_t p0 = (uint32_t)(s - __ldg(span0 + w)) * spanLen;
@@ -152,7 +138,7 @@ __global__ void __launch_bounds__(256) k_scan_spans_wide(const __grid_constant__
     const uint64_t nWarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
     const uint32_t k = t.k;
     for (uint64_t s = s0 + warp; s < s1; s += nWarps) {
-        const uint32_t w = window_of_span(span0, nWin, s);
+        const uint32_t w = dev::window_of_span(span0, nWin, s, lane);
         const uint64_t base = win[w].base;
         const uint32_t nPos = win[w].nPos;
         const uint32_t p0 = (uint32_t)(s - __ldg(span0 + w)) * spanLen;
@@ -200,7 +186,7 @@ __global__ void __launch_bounds__(kMzThreads, 3) k_scan_spans_mz(const __grid_co
     const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
     const uint64_t nWarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
     for (uint64_t s = s0 + warp; s < s1; s += nWarps) {
-        const uint32_t w = window_of_span(span0, nWin, s);
+        const uint32_t w = dev::window_of_span(span0, nWin, s, lane);
         const uint64_t base = win[w].base;
         const uint32_t nPos = win[w].nPos;
         const uint32_t p0 = (uint32_t)(s - __ldg(span0 + w)) * spanLen;

@@ -59,6 +59,24 @@ template <bool REVERSED = false> struct LaneFold {
     }
 };
 
+// The window that holds span s: the last w with span0[w] <= s (span0[0] = 0).
+// Every lane of the warp calls it with the same s. Each round probes 32 places
+// of what is left, so 1.5e7 windows take five dependent reads; a binary search
+// by all lanes alike took 24, most of the time of a span of few positions (30
+// Mbp at W = 27, k = 25: 32.8 ms with it, 19.6 with this).
+__device__ __forceinline__ uint32_t window_of_span(const uint32_t *__restrict__ span0, uint32_t nWin, uint64_t s,
+                                                   uint32_t lane)
+{
+    uint32_t lo = 0, left = nWin;
+    while (left > 1) {
+        const uint32_t step = (left + 31) / 32, at = lane * step;
+        const uint32_t last = 31 - __clz(__ballot_sync(FULL_MASK, at == 0 || (at < left && __ldg(span0 + lo + at) <= s)));
+        lo += last * step;
+        left = min(step, left - last * step);
+    }
+    return lo;
+}
+
 // Canonical code of the k-mer whose first base is packed base G, and whether
 // its k bases are all ACGT. Reads two sequence words and two mask words.
 __device__ __forceinline__ uint64_t canonical_at(const uint64_t *__restrict__ seq,
