@@ -292,8 +292,10 @@ uint32_t finish_lanes(const ScanPlan &p, uint64_t windows);
 // Positions per span for a reference (or a group of its windows) of `bases`:
 // the tuned length, or less where that would leave the GPU's warps without a
 // span (1 Mbp in spans of 2048 is 490 warps on 32 of 148 SMs, 51 us; in spans
-// of 128, 7800 warps), and cutting full windows evenly.
-uint32_t span_length(uint64_t bases, uint32_t tuned, uint32_t W, uint32_t k);
+// of 128, 7800 warps), and cutting full windows evenly. hash: the scan of a
+// hash-bucket table.
+uint32_t span_length(uint64_t bases, uint32_t tuned, uint32_t W, uint32_t k, bool hash);
+inline bool is_hash(uint32_t format) { return format == FMT_B8X32 || format == FMT_B6X40; }
 
 // Build the plan's host arrays for contigs `lens` starting at packed
 // offsets `baseOff`.
@@ -316,7 +318,7 @@ struct ibs_reference {
     std::vector<std::string> ids;       // contig ids when parsed from FASTA by the library
     uint64_t seqWords = 0, maskWords = 0;
     uint64_t *dSeq = nullptr, *dMask = nullptr;
-    ibs::ScanPlan plan;                 // cached for the last (W, k)
+    ibs::ScanPlan plans[2];             // cached for the last (W, k); [1]: spans of the hash-bucket scan
     ibs_window *dRows = nullptr;        // cached row buffer for ibs_scan
     uint64_t dRowsCap = 0;
     ibs::SegStats *dPanelSpans = nullptr; // panel scratch

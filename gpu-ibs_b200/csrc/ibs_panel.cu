@@ -752,7 +752,7 @@ static ibs_status panel_plan(ibs_panel_table *p, const ibs_reference *ref, uint3
     uint64_t bases = 0;
     for (uint64_t l : ref->lens)
         bases += l;
-    const uint32_t spanLen = span_length(bases, tuning().panel_span_len, W, p->geom.k);
+    const uint32_t spanLen = span_length(bases, tuning().panel_span_len, W, p->geom.k, false);
     if (p->planRef == ref && p->plan.W == W && p->plan.dWin && p->planLens == ref->lens &&
         p->plan.spanLen == spanLen && (pass_count(p) <= 1 || p->dMasks))
         return IBS_OK;

@@ -238,13 +238,17 @@ void ScanPlan::release()
 // 24 warps a SM are what the scan kernels keep resident; with four spans each
 // they even out (16 Mbp of wide keys: 377 us with two, 345 with four), but short
 // spans have more to sum up (1 Mbp: 50 us with one span of 256 a warp, 57 with two
-// of 128). Below 128 positions a span has less than one block of the
-// minimizer-line scan. Then the length that cuts a full window into equal spans
-// of whole blocks: 50 kbp in spans of 4096 would leave one of 824.
-uint32_t span_length(uint64_t bases, uint32_t tuned, uint32_t W, uint32_t k)
+// of 128). The hash-bucket scan has 32 warps a SM, in CTAs of 16 that wait for
+// their slowest, and no keys to locate again at a span's edge: eight each (80
+// Mbp at k = 25: 1642 us with three spans a warp, 1510 with eight; the
+// minimizer-line scan of 20 Mbp 158 us with four, 177 with eight). Below 128
+// positions a span has less than one block of the minimizer-line scan. Then the
+// length that cuts a full window into equal spans of whole blocks: 50 kbp in
+// spans of 4096 would leave one of 824.
+uint32_t span_length(uint64_t bases, uint32_t tuned, uint32_t W, uint32_t k, bool hash)
 {
-    const uint64_t warps = (uint64_t)sm_count() * 24;
-    while (tuned >= 256 && tuned % 256 == 0 && bases / tuned < warps * (tuned > 512 ? 4 : 1))
+    const uint64_t sms = (uint64_t)sm_count(), many = sms * (hash ? 32 * 8 : 24 * 4);
+    while (tuned >= 256 && tuned % 256 == 0 && bases / tuned < (tuned > 512 ? many : sms * 24))
         tuned /= 2;
     const uint32_t blocks = (W - k + 1 + 127) / 128, want = tuned / 128;
     const uint32_t n = (blocks + want - 1) / want; // spans a window
@@ -701,7 +705,8 @@ extern "C" void ibs_reference_free(ibs_reference *r)
         DeviceGuard guard(r->device);
         if (r->stream)
             cudaStreamSynchronize(r->stream);
-        r->plan.release();
+        for (ScanPlan &p : r->plans)
+            p.release();
         cudaFree(r->dSeq);
         cudaFree(r->dMask);
         cudaFree(r->dRows);
@@ -713,21 +718,27 @@ extern "C" void ibs_reference_free(ibs_reference *r)
 }
 
 // Makes r->plan describe (W, k); allocates and uploads on a change.
-static ibs_status ensure_plan(ibs_reference *r, uint32_t W, uint32_t k)
+// The reference's plan for (W, k) and a kind of table, made where no cached
+// plan has that span length.
+static ibs_status ensure_plan(ibs_reference *r, uint32_t W, uint32_t k, bool hash, ScanPlan **out)
 {
-    ScanPlan &p = r->plan;
     uint64_t bases = 0;
     for (uint64_t l : r->lens)
         bases += l;
-    const uint32_t spanLen = span_length(bases, tuning().span_len, W, k);
-    if (p.dWin && p.W == W && p.k == k && p.spanLen == spanLen)
-        return IBS_OK;
+    const uint32_t spanLen = span_length(bases, tuning().span_len, W, k, hash);
+    for (ScanPlan &p : r->plans)
+        if (p.dWin && p.W == W && p.k == k && p.spanLen == spanLen) {
+            *out = &p;
+            return IBS_OK;
+        }
     IBS_CUDA(cudaStreamSynchronize(r->stream), "plan sync");
+    ScanPlan &p = r->plans[hash];
     p.release();
     plan_windows(p, r->lens, r->baseOff, W, k, spanLen);
     ibs_status s = upload_plan(p, r->stream);
     if (s != IBS_OK)
         p.release();
+    *out = &p;
     return s;
 }
 
@@ -765,15 +776,16 @@ extern "C" ibs_status ibs_scan_async(ibs_table *t, ibs_reference *ref, uint32_t 
     if (s != IBS_OK)
         return s;
     DeviceGuard guard(t->device);
-    s = ensure_plan(ref, W, t->geom.k);
+    ScanPlan *plan = nullptr;
+    s = ensure_plan(ref, W, t->geom.k, is_hash(t->geom.format), &plan);
     if (s != IBS_OK)
         return s;
     IBS_CUDA(cudaStreamSynchronize(ref->stream), "plan sync");
     cudaStream_t st = (cudaStream_t)stream;
-    s = launch_scan(t, ref->dSeq, ref->dMask, ref->plan, 0, ref->plan.nSpans, st);
+    s = launch_scan(t, ref->dSeq, ref->dMask, *plan, 0, plan->nSpans, st);
     if (s != IBS_OK)
         return s;
-    return launch_finalize(ref->plan, t->geom.k, rows_dev, st);
+    return launch_finalize(*plan, t->geom.k, rows_dev, st);
 }
 
 extern "C" ibs_status ibs_scan(ibs_table *t, ibs_reference *ref, uint32_t W, ibs_window *rows,
@@ -784,10 +796,11 @@ extern "C" ibs_status ibs_scan(ibs_table *t, ibs_reference *ref, uint32_t W, ibs
     if (s != IBS_OK)
         return s;
     DeviceGuard guard(t->device);
-    s = ensure_plan(ref, W, t->geom.k);
+    ScanPlan *plan = nullptr;
+    s = ensure_plan(ref, W, t->geom.k, is_hash(t->geom.format), &plan);
     if (s != IBS_OK)
         return s;
-    const uint64_t nWin = ref->plan.nWin;
+    const uint64_t nWin = plan->nWin;
     if (ref->dRowsCap < nWin) {
         cudaFree(ref->dRows);
         ref->dRows = nullptr;
@@ -796,10 +809,10 @@ extern "C" ibs_status ibs_scan(ibs_table *t, ibs_reference *ref, uint32_t W, ibs
                  "row buffer alloc");
         ref->dRowsCap = nWin;
     }
-    s = launch_scan(t, ref->dSeq, ref->dMask, ref->plan, 0, ref->plan.nSpans, ref->stream);
+    s = launch_scan(t, ref->dSeq, ref->dMask, *plan, 0, plan->nSpans, ref->stream);
     if (s != IBS_OK)
         return s;
-    s = launch_finalize(ref->plan, t->geom.k, ref->dRows, ref->stream);
+    s = launch_finalize(*plan, t->geom.k, ref->dRows, ref->stream);
     if (s != IBS_OK)
         return s;
     if (nWin)
@@ -830,7 +843,11 @@ extern "C" ibs_status ibs_scan_panel(ibs_table *const *tables, uint32_t n, ibs_r
     if (s != IBS_OK)
         return s;
     DeviceGuard guard(ref->device);
-    s = ensure_plan(ref, W, k);
+    bool hash = true; // spans of the minimizer-line scan as soon as one table takes it
+    for (uint32_t i = 0; i < n; ++i)
+        hash = hash && is_hash(tables[i]->geom.format);
+    ScanPlan *plan = nullptr;
+    s = ensure_plan(ref, W, k, hash, &plan);
     if (s != IBS_OK)
         return s;
     const uint64_t need = nWin * n;
@@ -842,7 +859,7 @@ extern "C" ibs_status ibs_scan_panel(ibs_table *const *tables, uint32_t n, ibs_r
                  "row buffer alloc");
         ref->dRowsCap = need;
     }
-    s = launch_panel(tables, n, ref->dSeq, ref->dMask, ref->plan, ref->dRows, ref->plan.dSpans,
+    s = launch_panel(tables, n, ref->dSeq, ref->dMask, *plan, ref->dRows, plan->dSpans,
                      ref->stream);
     if (s != IBS_OK)
         return s;
@@ -977,7 +994,8 @@ extern "C" ibs_status ibs_scan_packed(ibs_table *t, const uint64_t *seq2bit,
     std::vector<uint64_t> lv(lens, lens + n);
     ScanPlan &p = ws.plan;
     // the windows go in groups, the first a 128th of the reference
-    plan_windows(p, lv, off, W, k, span_length((seqWords - 1) * 32 / 8, tuning().span_len, W, k));
+    plan_windows(p, lv, off, W, k, span_length((seqWords - 1) * 32 / 8, tuning().span_len, W, k,
+                                         is_hash(t->geom.format)));
     if (p.nSpans > ws.spansCap || !p.dSpans) {
         cudaFree(p.dSpans);
         p.dSpans = nullptr;

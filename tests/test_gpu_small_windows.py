@@ -1,6 +1,7 @@
 """Rows of windows of very different span counts: groups of 1 to 32 lanes finish
 a window, and a window of many spans among hundreds of thousands of one-span
-windows is finished by fewer lanes than it has spans."""
+windows is finished by fewer lanes than it has spans; and tables of both kinds
+on one reference, whose spans differ in length."""
 import numpy as np
 import pytest
 
@@ -72,3 +73,28 @@ def test_long_windows_among_very_many_short_ones():
         assert np.array_equal(rows[-second:], alone[first:first + second])
         assert np.array_equal(rows[first:-second], np.tile(alone[first + second:], n_short // 10))
         assert rows["observed_kmers"].sum() > 0
+
+
+def test_tables_of_both_kinds_in_turn():
+    """24 Mbp: spans of 512 positions for hash buckets, 1024 for minimizer lines."""
+    import torch
+    spec = ib.RefSpec(seed=77, lens=[20_000_000, 4_000_001], n_frac=0.003, n_run=(1, 300))
+    sw, mw = spec.packed_words()
+    seq, mask = (torch.empty(n, dtype=torch.int64, device="cuda") for n in (sw, mw))
+    spec.reference_device(seq, mask)
+    smp = ib.SampleSpec(seed=78, k=K, class_rate=(0.001, 0.03), class_prob=(0.5, 0.5), block_len=100_000,
+                        random_frac=0.05)
+    cap = smp.codes_device_bound(spec, seq, mask)
+    codes = torch.empty(cap, dtype=torch.int64, device="cuda")
+    n = smp.codes_device(spec, seq, mask, codes, cap)
+    ref = ib.Reference(seq, mask, spec.lens, on_device=True)
+    hashed, lined = (ib.Table.from_codes(codes, n, K, on_device=True, force_format=f) for f in (5, 4))
+    other = ib.Table.from_codes(codes, n // 2, K, on_device=True, force_format=5)
+    for W in (5000, 50_000):
+        want, half = ib.scan(hashed, ref, W), ib.scan(other, ref, W)
+        assert 0 < half["observed_kmers"].sum() < want["observed_kmers"].sum()
+        for _ in range(2):
+            assert np.array_equal(ib.scan(lined, ref, W), want)
+            assert np.array_equal(ib.scan(hashed, ref, W), want)
+        for tables, rows in (([hashed, other], [want, half]), ([other, lined], [half, want])):
+            assert np.array_equal(np.asarray(ib.scan_panel(tables, ref, W)).reshape(2, -1), np.stack(rows))
