@@ -53,9 +53,14 @@ constexpr uint64_t kFinCap = 1ull << 20;   // (request, window) rows finalized p
 constexpr uint64_t kRowPool = 4ull << 20;  // rows of admitted requests (24 B each): 96 MiB
 constexpr uint32_t kMaxGroups = 4096;
 constexpr int kDepth = 4;                  // iterations (batches) in flight
-constexpr int kServeNB = 2;                // blocks in flight per lane of the single-table kernel (64
-                                           // registers, four CTAs of 256 per SM) and of the persistent
-                                           // kernel (80 registers without spills, three CTAs per SM)
+// Blocks in flight per lane of a hash-bucket table's items in the single-table
+// kernel (64 registers, four CTAs of 256 per SM) and the persistent kernel (80,
+// three CTAs). The minimizer path spills at both: 176 to 224 bytes at k <= 27 and
+// 120 to 136 above in the former, 136 to 292 in the latter (ptxas -v), some of it
+// the ticket's state around an item. Against kernels without those spills, but
+// with a run-time k, whole-genome requests of six k = 25 samples went from 4.6 to
+// 3.5 ms (one launch an iteration) and from 5.4 to 4.2 ms (persistent).
+constexpr int kServeNB = 2;
 
 struct WorkItem {
     uint64_t base;   // packed base offset of the window's first base
@@ -71,6 +76,70 @@ struct FinItem {
     int32_t start, end;
     uint64_t row;    // row slot
 };
+
+// Positions [p0, p1) of a window over a hash-bucket table, one bucket load per
+// position (16-byte halves: ptxas 12.9 crashes on 32-byte loads in functions
+// kept out of line, as serve_hash_span is).
+template <int NB>
+__device__ __forceinline__ SegStats hash_span(const TableView &t, const uint64_t *__restrict__ seq,
+                                                 const uint64_t *__restrict__ mask, uint64_t base, uint32_t p0,
+                                                 uint32_t p1, uint32_t lane)
+{
+    const uint32_t k = t.g.k;
+    const uint64_t kmask = key_mask(2 * k);
+    const uint64_t kbits = (1ull << k) - 1;
+    const bool b8 = t.g.format == FMT_B8X32;
+    dev::LaneFold<> fold;
+    for (uint32_t p = p0; p < p1; p += 32 * NB) {
+        uint4 v0[NB], v1[NB];
+        uint64_t code[NB], fp[NB];
+        bool valid[NB];
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+            const uint32_t q = p + 32 * b + lane;
+            const bool in = q < p1;
+            const uint64_t G = base + (in ? q : p0);
+            bool acgt;
+            code[b] = dev::canonical_at(seq, mask, G, k, kmask, kbits, acgt);
+            valid[b] = in && acgt;
+            const uint64_t h = perm_hash(code[b], t.g.bits);
+            const uint64_t r = bucket_of(h, t.g);
+            fp[b] = fp_of(h, t.g);
+            if (valid[b]) {
+                v0[b] = __ldg(t.buckets + 2 * r);
+                v1[b] = __ldg(t.buckets + 2 * r + 1);
+            } else {
+                v0[b] = make_uint4(0, 0, 0, 0);
+                v1[b] = make_uint4(0, 0, 0, 0);
+            }
+        }
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+            bool hit = false;
+            if (valid[b]) {
+                const uint32_t m = b8 ? bucket_match<FMT_B8X32>(v0[b], v1[b], fp[b])
+                                      : bucket_match<FMT_B6X40>(v0[b], v1[b], fp[b]);
+                hit = m == 1u || (m == 2u && stash_lookup(t, code[b]));
+            }
+            const uint32_t V = __ballot_sync(dev::FULL_MASK, valid[b]);
+            const uint32_t H = __ballot_sync(dev::FULL_MASK, hit);
+            fold.push(V, H, lane, (int)k);
+        }
+    }
+    return fold.finish((int)k);
+}
+
+// The same out of line, so that its loop has the registers to itself: beside the
+// minimizer path it shared that one's spills in the persistent kernel (four k =
+// 25 samples in hash sectors, 20 whole-contig requests of 40 Mbp: 4.02 to 4.10 ms
+// inlined, 3.94 to 4.02 out of line, 3.93 in a kernel without the located blocks).
+template <int NB>
+__device__ __noinline__ SegStats serve_hash_span(const TableView &t, const uint64_t *__restrict__ seq,
+                                                 const uint64_t *__restrict__ mask, uint64_t base, uint32_t p0,
+                                                 uint32_t p1, uint32_t lane)
+{
+    return hash_span<NB>(t, seq, mask, base, p0, p1, lane);
+}
 
 // One work item over a single-sample table, by one warp: the summary of
 // positions [p0, p1) of its window goes to sums[it.out]. Minimizer-line
@@ -100,48 +169,8 @@ __device__ __forceinline__ void serve_single_item(const WorkItem &it, const Tabl
             return;
         }
     }
-    const uint32_t k = t.g.k;
-    const uint64_t kmask = key_mask(2 * k);
-    const uint64_t kbits = (1ull << k) - 1;
-    const bool b8 = t.g.format == FMT_B8X32;
-    dev::LaneFold<> fold;
-    for (uint32_t p = it.p0; p < it.p1; p += 32 * NB) {
-        uint4 v0[NB], v1[NB];
-        uint64_t code[NB], fp[NB];
-        bool valid[NB];
-#pragma unroll
-        for (int b = 0; b < NB; ++b) {
-            const uint32_t q = p + 32 * b + lane;
-            const bool in = q < it.p1;
-            const uint64_t G = it.base + (in ? q : it.p0);
-            bool acgt;
-            code[b] = dev::canonical_at(seq, mask, G, k, kmask, kbits, acgt);
-            valid[b] = in && acgt;
-            const uint64_t h = perm_hash(code[b], t.g.bits);
-            const uint64_t r = bucket_of(h, t.g);
-            fp[b] = fp_of(h, t.g);
-            if (valid[b]) {
-                v0[b] = __ldg(t.buckets + 2 * r);
-                v1[b] = __ldg(t.buckets + 2 * r + 1);
-            } else {
-                v0[b] = make_uint4(0, 0, 0, 0);
-                v1[b] = make_uint4(0, 0, 0, 0);
-            }
-        }
-#pragma unroll
-        for (int b = 0; b < NB; ++b) {
-            bool hit = false;
-            if (valid[b]) {
-                const uint32_t m = b8 ? bucket_match<FMT_B8X32>(v0[b], v1[b], fp[b])
-                                      : bucket_match<FMT_B6X40>(v0[b], v1[b], fp[b]);
-                hit = m == 1u || (m == 2u && stash_lookup(t, code[b]));
-            }
-            const uint32_t V = __ballot_sync(dev::FULL_MASK, valid[b]);
-            const uint32_t H = __ballot_sync(dev::FULL_MASK, hit);
-            fold.push(V, H, lane, (int)k);
-        }
-    }
-    const SegStats acc = fold.finish((int)k);
+    const SegStats acc = K ? serve_hash_span<NB>(t, seq, mask, it.base, it.p0, it.p1, lane)
+                           : hash_span<NB>(t, seq, mask, it.base, it.p0, it.p1, lane);
     if (lane == 0)
         sums[it.out] = acc;
 }
