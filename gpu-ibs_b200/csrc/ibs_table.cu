@@ -252,30 +252,32 @@ __global__ void k_count_left(const uint64_t *__restrict__ list, const unsigned l
 // Settles the listed keys: a B8x32 bucket's only one takes slot 7; otherwise
 // a minimizer line's go to the line's free slots, the partner sector's first
 // (a sector's slot 7 only where that sector has no listed keys of its own),
-// and what is left, as every listed key of a hash bucket, to the stash list.
-// The home bucket's marker says how far.
-__global__ void k_spill(const uint64_t *__restrict__ list, const unsigned long long *__restrict__ listN,
-                        uint64_t listCap, TableGeom g, const uint32_t *__restrict__ left,
-                        uint32_t *__restrict__ words, uint64_t *__restrict__ stashList,
+// and what is left, as every listed key of a hash bucket, stays in the list for
+// the stash (the others' entries become STASH_EMPTY, which is no key). The home
+// bucket's marker says how far.
+__global__ void k_spill(uint64_t *__restrict__ list, const unsigned long long *__restrict__ listN, uint64_t listCap,
+                        TableGeom g, const uint32_t *__restrict__ left, uint32_t *__restrict__ words,
                         unsigned long long *__restrict__ stashN)
 {
     const uint64_t n = *listN <= listCap ? *listN : 0;
     const bool b8 = g.format == FMT_B8X32 || g.format == FMT_MZ8, mz = is_mz(g.format);
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
          i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t code = mz ? list[i] & ~(mz::kSecondPlace | mz::kNoPlace) : list[i];
-        if (mz && (list[i] & mz::kNoPlace)) {
-            stashList[atomicAdd(stashN, 1ull)] = code;
+        const uint64_t entry = list[i], code = mz ? entry & ~(mz::kSecondPlace | mz::kNoPlace) : entry;
+        if (mz && (entry & mz::kNoPlace)) {
+            list[i] = code;
+            atomicAdd(stashN, 1ull);
             continue;
         }
         uint64_t rr[2], ff[2];
         locate_key(code, g, rr, ff);
-        const uint32_t a = mz ? (uint32_t)(list[i] >> 63) : 0; // which of its places
+        const uint32_t a = mz ? (uint32_t)(entry >> 63) : 0; // which of its places
         const uint64_t r = a ? rr[1] : rr[0], fp = a ? ff[1] : ff[0];
         uint32_t *home = words + r * 8;
         auto left_of = [&](uint64_t x) { return (left[x >> 4] >> (2 * (x & 15))) & 3u; };
         if (b8 && left_of(r) == 1u) {
             home[7] = (uint32_t)fp;
+            list[i] = STASH_EMPTY;
             continue;
         }
         uint32_t reach = 3;
@@ -284,8 +286,9 @@ __global__ void k_spill(const uint64_t *__restrict__ list, const unsigned long l
             if (b8 ? claim8(w, (uint32_t)fp, left_of(r ^ d) ? 7 : 8) : claim6(w, fp))
                 reach = d == 1 ? 1 : 2;
         }
+        list[i] = reach == 3 ? code : STASH_EMPTY;
         if (reach == 3)
-            stashList[atomicAdd(stashN, 1ull)] = code;
+            atomicAdd(stashN, 1ull);
         if (!mz)
             reach = 1; // hash buckets: the marker (B8_OVERFLOW, flag bit 0) means the stash
         if (b8)
@@ -300,7 +303,7 @@ __global__ void k_stash(const uint64_t *__restrict__ list, uint64_t n, uint64_t 
 {
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
          i += (uint64_t)gridDim.x * blockDim.x)
-        if (!stash_insert(stash, stashBuckets, list[i]))
+        if (list[i] != STASH_EMPTY && !stash_insert(stash, stashBuckets, list[i]))
             atomicExch(err, 1);
 }
 
@@ -416,25 +419,26 @@ static ibs_status build_from_device_codes(ibs_table *t, const uint64_t *dCodes, 
     t->deviceBytes = nb * 32;
     uint32_t *words = reinterpret_cast<uint32_t *>(t->buckets);
     // scratch in one allocation: counts (listed keys, keys for the stash, error),
-    // the list, the stash's list, and two bits a bucket
+    // the list, and two bits a bucket
     const uint64_t leftBytes = b8 ? (nb + 15) / 16 * 4 : 0;
     std::unique_ptr<uint8_t, cudaError_t (*)(void *)> scratch(nullptr, cudaFree);
     unsigned long long *dCounts = nullptr;
-    uint64_t *list = nullptr, *stashList = nullptr;
+    uint64_t *list = nullptr;
     uint32_t *left = nullptr;
     unsigned long long counts[2] = {0, 0};
     // about 2% of the keys find no slot at the default loads; a table that
-    // leaves more (a forced load, many duplicates) is filled again with a
-    // list of the size that it then needs and as much again
+    // leaves more (a forced load, many duplicates) is filled again with a list
+    // of the size that it then needs (which of several equal keys are listed
+    // can differ from pass to pass), at most of every place of every key
     uint64_t listCap = n / 16 + 4096;
+    const uint64_t most = n * (is_mz(g.format) ? 2 : 1) + 4096;
     for (int attempt = 0;; ++attempt) {
         void *mem = nullptr;
-        IBS_CUDA(cudaMalloc(&mem, 32 + listCap * 16 + leftBytes), "table build scratch");
+        IBS_CUDA(cudaMalloc(&mem, 32 + listCap * 8 + leftBytes), "table build scratch");
         scratch.reset(static_cast<uint8_t *>(mem));
         dCounts = static_cast<unsigned long long *>(mem);
         list = reinterpret_cast<uint64_t *>(dCounts + 4);
-        stashList = list + listCap;
-        left = reinterpret_cast<uint32_t *>(stashList + listCap);
+        left = reinterpret_cast<uint32_t *>(list + listCap);
         IBS_CUDA(cudaMemsetAsync(t->buckets, b8 ? 0xff : 0x00, nb * 32, 0), "table init");
         IBS_CUDA(cudaMemsetAsync(dCounts, 0, 32, 0), "table build scratch");
         if (n) {
@@ -445,18 +449,14 @@ static ibs_status build_from_device_codes(ibs_table *t, const uint64_t *dCodes, 
                 k_count_left<<<grid_for(listCap, 256), 256>>>(list, dCounts, listCap, g, left);
                 IBS_LAUNCHED();
             }
-            k_spill<<<grid_for(listCap, 256), 256>>>(list, dCounts, listCap, g, left, words, stashList, dCounts + 1);
+            k_spill<<<grid_for(listCap, 256), 256>>>(list, dCounts, listCap, g, left, words, dCounts + 1);
             IBS_LAUNCHED();
         }
         IBS_CUDA(cudaMemcpy(counts, dCounts, 16, cudaMemcpyDeviceToHost), "table build");
         if (counts[0] <= listCap)
             break;
-        if (attempt == 3) {
-            set_error("table build: the list of keys without a slot keeps growing");
-            return IBS_ERR_CAPACITY;
-        }
         scratch.reset();
-        listCap = 2 * counts[0];
+        listCap = std::min<uint64_t>(attempt ? 2 * counts[0] : counts[0] + counts[0] / 16 + 4096, most);
     }
     t->stashKeys = counts[1];
     if (!counts[1])
@@ -466,7 +466,7 @@ static ibs_status build_from_device_codes(ibs_table *t, const uint64_t *dCodes, 
     g.stashBuckets = stashBuckets;
     t->deviceBytes += stashBuckets * 32;
     IBS_CUDA(cudaMemsetAsync(t->stash, 0xff, stashBuckets * 32, 0), "stash alloc");
-    k_stash<<<grid_for(counts[1], 256), 256>>>(stashList, counts[1], t->stash, stashBuckets,
+    k_stash<<<grid_for(counts[0], 256), 256>>>(list, counts[0], t->stash, stashBuckets,
                                                reinterpret_cast<int *>(dCounts + 2));
     IBS_LAUNCHED();
     int herr = 0;

@@ -170,7 +170,8 @@ ibs_status build_wide(ibs_table *t, const ulonglong2 *dCodes, uint64_t n, uint32
         t->wide.nLevels = L + 1;
         bytes += lines * kSlots * sizeof(ulonglong2);
         // about 1% of the keys find their line full at the default load; a level
-        // that leaves more is filled again with room for as many
+        // that leaves more is filled again with room for as many (a line of c keys
+        // leaves c - 8, whichever they are)
         std::unique_ptr<DevPtr<ulonglong2>> next(new DevPtr<ulonglong2>);
         unsigned long long over = 0;
         for (uint64_t cap = nCur / 16 + 4096;;) {
@@ -184,7 +185,7 @@ ibs_status build_wide(ibs_table *t, const ulonglong2 *dCodes, uint64_t n, uint32
             IBS_CUDA(cudaMemcpy(&over, dOver.p, sizeof over, cudaMemcpyDeviceToHost), "wide table place");
             if (over <= cap)
                 break;
-            cap = nCur;
+            cap = over;
             next.reset(new DevPtr<ulonglong2>);
         }
         if (L == 0)

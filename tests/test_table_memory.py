@@ -57,3 +57,46 @@ def test_joint_lines_take_no_more_than_hash_sectors(k, few, many):
     pt = ib.PanelTable(k, few, keys_per_bucket=3.0)
     assert pt.info()[0].format == 3
     pt.close()
+
+
+def _leave(nbytes):
+    """Takes all the device's free memory but nbytes."""
+    import torch
+    torch.cuda.empty_cache()
+    free, _ = torch.cuda.mem_get_info()
+    return torch.empty(free - nbytes, dtype=torch.uint8, device="cuda")
+
+
+@pytest.mark.gpu
+def test_dense_tables_build_with_little_scratch():
+    """Loads at which four keys in ten find no slot: the build's scratch is 8
+    bytes for each of those (16 for a wide key), not for every key."""
+    import torch
+    n, kpb = 40_000_000, 12.0
+    codes = torch.randint(0, 1 << 62, (n,), device="cuda")
+    table = ib.table_bytes_for(n, 31, force_format=5, keys_per_bucket=kpb)
+
+    def build():
+        t = ib.Table.from_codes(codes, n, 31, on_device=True, force_format=5, keys_per_bucket=kpb)
+        info = t.info()
+        assert info.format in (1, 2) and 0.3 * n < info.stash_keys < 0.6 * n
+        assert info.device_bytes < table + (600 << 20)
+        t.close()
+
+    build()
+    held = _leave(table + (480 << 20))  # the table, its 256 MiB of stash and 5.9 bytes a key
+    build()
+    del held
+    rng = np.random.default_rng(1)
+    m = 10_000_000
+    lo, hi = rng.integers(0, 1 << 62, m).astype(np.uint64), rng.integers(0, 1 << 17, m).astype(np.uint64)
+
+    def build_wide():
+        ib.Table.from_codes128(lo, hi, 41, keys_per_bucket=7.9).close()
+
+    build_wide()
+    wide = int(m / 7.9 * 128)
+    held = _leave(16 * m + wide + wide // 2 + (60 << 20))  # codes, level 0, the later levels, 6 bytes a key
+    build_wide()
+    del held
+    torch.cuda.empty_cache()
