@@ -21,7 +21,7 @@ constexpr uint64_t kStashProbe = 64;
 // sectors' 3)
 constexpr double kPmKeysPerSector = 1.5;
 constexpr double kPm6KeysPerSector = 1.2; // the same share of a sector's four slots
-constexpr uint64_t kBuildChunk = 1ull << 27; // places of keys per build step (1 GiB of scratch each way)
+constexpr uint64_t kBuildChunk = 1ull << 27; // keys' places per build step (1 GiB of scratch each way)
 
 // Slot of fingerprint (or slot value) fp among sector w's first count slots,
 // or -1. wide: four 40-bit slot values (PM6).
@@ -89,8 +89,10 @@ __device__ __forceinline__ bool claim_slot(uint32_t *w, uint64_t fp, uint32_t bi
 // lookup races with an insert of the same key. A key is looked for where
 // phase B would have put it: its home sector, then (PM, flagged) the line's
 // others, then (flagged) the stash; a key with two places, at each.
+// nPending counts every place without a slot, also those past cap that are not
+// written (finding again changes nothing: the bit is set already).
 __global__ void k_find(View t, uint32_t *words, unsigned long long *stashWords, const uint64_t *codes,
-                       uint64_t n, uint32_t bit, uint64_t *pending, unsigned long long *nPending)
+                       uint64_t n, uint32_t bit, uint64_t *pending, unsigned long long *nPending, uint64_t cap)
 {
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
@@ -132,9 +134,9 @@ __global__ void k_find(View t, uint32_t *words, unsigned long long *stashWords, 
             if (lane == 0)
                 base = atomicAdd(nPending, (unsigned long long)__popc(ballot));
             base = __shfl_sync(0xffffffffu, base, 0);
-            if (miss)
-                pending[base + __popc(ballot & ((1u << lane) - 1u))] =
-                    code | (!places ? mz::kNoPlace : a ? mz::kSecondPlace : 0ull);
+            base += __popc(ballot & ((1u << lane) - 1u));
+            if (miss && base < cap)
+                pending[base] = code | (!places ? mz::kNoPlace : a ? mz::kSecondPlace : 0ull);
         }
     }
 }
@@ -600,25 +602,36 @@ static ibs_status panel_add_device_codes(ibs_panel_table *p, const uint64_t *dCo
         cudaGraphExecDestroy(p->graph);
         p->graph = nullptr;
     }
-    // keys go in chunks, so the build's scratch stays small next to the table
+    // keys go in chunks, so the build's scratch stays small next to the table. On
+    // minimizer lines a key can have two places, but few have (short tandem
+    // repeats, reverse-palindromic minimizers): the lists have room for an
+    // eighth more places than keys, and a chunk with more is begun again with half
+    // as many keys as they hold. (With lists of two places a key the eight samples
+    // of 20 Mbp at k = 21 took 18.1 ms to add, 16.3 so.)
+    const bool lines = is_joint_mz(p->geom.format);
+    const uint64_t chunk = std::max<uint64_t>(1, std::min<uint64_t>(n, lines ? kBuildChunk / 9 * 8 : kBuildChunk));
+    const uint64_t cap = lines ? chunk + chunk / 8 + 4096 : chunk;
     uint64_t *pending = nullptr, *failed = nullptr;
-    const uint64_t places = is_joint_mz(p->geom.format) ? 2 : 1; // most places a key has
-    const uint64_t chunk = std::max<uint64_t>(1, std::min<uint64_t>(n, kBuildChunk / places));
-    IBS_CUDA(cudaMalloc(&pending, chunk * places * 8), "panel pending alloc");
+    IBS_CUDA(cudaMalloc(&pending, cap * 8), "panel pending alloc");
     std::unique_ptr<uint64_t, cudaError_t (*)(void *)> g1(pending, cudaFree);
-    IBS_CUDA(cudaMalloc(&failed, chunk * places * 8), "panel pending alloc");
+    IBS_CUDA(cudaMalloc(&failed, cap * 8), "panel pending alloc");
     std::unique_ptr<uint64_t, cudaError_t (*)(void *)> g2(failed, cudaFree);
     unsigned long long *cnt = p->dCounters; // [0] pending, [2] failed
-    for (uint64_t c0 = 0; c0 < n; c0 += chunk) {
-        const uint64_t m = std::min<uint64_t>(chunk, n - c0);
-        IBS_CUDA(cudaMemset(cnt, 0, 8), "panel build");
-        View v = p->view();
-        k_find<<<grid_for(m), 256>>>(v, reinterpret_cast<uint32_t *>(p->buckets),
-                                     reinterpret_cast<unsigned long long *>(p->stash), dCodes + c0, m, bit,
-                                     pending, cnt);
-        IBS_LAUNCHED();
+    for (uint64_t c0 = 0, m = 0; c0 < n; c0 += m) {
+        m = std::min<uint64_t>(chunk, n - c0);
         unsigned long long nPend = 0;
-        IBS_CUDA(cudaMemcpy(&nPend, cnt, 8, cudaMemcpyDeviceToHost), "panel build find");
+        for (;;) {
+            IBS_CUDA(cudaMemset(cnt, 0, 8), "panel build");
+            View v = p->view();
+            k_find<<<grid_for(m), 256>>>(v, reinterpret_cast<uint32_t *>(p->buckets),
+                                         reinterpret_cast<unsigned long long *>(p->stash), dCodes + c0, m, bit,
+                                         pending, cnt, cap);
+            IBS_LAUNCHED();
+            IBS_CUDA(cudaMemcpy(&nPend, cnt, 8, cudaMemcpyDeviceToHost), "panel build find");
+            if (nPend <= cap)
+                break;
+            m = cap / 2; // two places each fit
+        }
         const uint64_t *todo = pending;
         for (int round = 0; nPend; ++round) {
             if (round > 40) { // each round doubles the stash: 2^40 x its start is out of reach
