@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <atomic>
+#include <cmath>
 #include <cstdint>
 #include <mutex>
 #include <string>
@@ -288,6 +289,21 @@ struct ScanPlan {
 // that leaves lanes of the GPU idle (a few long contigs among many short ones),
 // as many as there are on average otherwise.
 uint32_t finish_lanes(const ScanPlan &p, uint64_t windows);
+
+// Expected fraction of keys beyond a bucket's slots when the keys per bucket are
+// Poisson(lam).
+inline double overflow_fraction(double lam, int slots)
+{
+    if (lam <= 0)
+        return 0;
+    double p = std::exp(-lam), over = 0;
+    for (int x = 0; x < 400; ++x) {
+        if (x > slots)
+            over += (x - slots) * p;
+        p *= lam / (x + 1);
+    }
+    return over / lam;
+}
 
 // Positions per span for a reference (or a group of its windows) of `bases`:
 // the tuned length, or less where that would leave the GPU's warps without a

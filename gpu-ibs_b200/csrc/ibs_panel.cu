@@ -416,21 +416,6 @@ int grid_for(uint64_t n)
     return (int)std::max<uint64_t>(1, std::min<uint64_t>((n + 255) / 256, (uint64_t)sm_count() * 16));
 }
 
-// Expected fraction of keys beyond a bucket's kSlots slots when the keys per
-// bucket are Poisson(lam).
-double overflow_fraction(double lam)
-{
-    if (lam <= 0)
-        return 0;
-    double p = std::exp(-lam), over = 0;
-    for (int x = 0; x < 400; ++x) {
-        if (x > (int)kSlots)
-            over += (x - (int)kSlots) * p;
-        p *= lam / (x + 1);
-    }
-    return over / lam;
-}
-
 uint64_t next_pow2(uint64_t x)
 {
     uint64_t p = 1;
@@ -532,7 +517,7 @@ extern "C" ibs_status ibs_panel_table_create(uint32_t k, uint64_t expected_keys,
         p->stashBuckets = fmt == FMT_PANEL_MZ6 ? lineStash(kPm6KeysPerSector, kPm6KeysPerSector)
                                                : lineStash(lamPm, kPmKeysPerSector);
     } else {
-        const double over = (double)expected_keys * overflow_fraction((double)expected_keys / (double)nb);
+        const double over = (double)expected_keys * overflow_fraction((double)expected_keys / (double)nb, kSlots);
         p->stashBuckets = next_pow2(std::max<uint64_t>(1u << 12, (uint64_t)(over * 0.75) + 1));
     }
     g.stashBuckets = p->stashBuckets;

@@ -9,6 +9,8 @@
 // codes, which the build then hashes into 32-byte buckets.
 #include "ibs_internal.cuh"
 
+#include <cooperative_groups.h>
+
 #include <chrono>
 #include <cstdio>
 #include <cstring>
@@ -206,6 +208,17 @@ __device__ __forceinline__ bool claim6(uint32_t *w, uint64_t fp)
     return false;
 }
 
+// A place in a list for each lane that calls it, one atomic for all of them
+// (with one each, 66M keys at 8 a bucket took 7.7 ms to build, so 6.2).
+__device__ __forceinline__ unsigned long long list_place(unsigned long long *listN)
+{
+    const auto lanes = cooperative_groups::coalesced_threads();
+    unsigned long long at = 0;
+    if (lanes.thread_rank() == 0)
+        at = atomicAdd(listN, (unsigned long long)lanes.size());
+    return lanes.shfl(at, 0) + lanes.thread_rank();
+}
+
 // Slot 7 of a B8x32 bucket stays free in this pass: it becomes a key's when
 // one key is left over, or the marker when there are more.
 __global__ void k_fill(const uint64_t *__restrict__ codes, uint64_t n, TableGeom g, uint32_t *__restrict__ words,
@@ -221,7 +234,7 @@ __global__ void k_fill(const uint64_t *__restrict__ codes, uint64_t n, TableGeom
             const uint64_t r = a ? rr[1] : rr[0], fp = a ? ff[1] : ff[0];
             if (places && (b8 ? claim8(words + r * 8, (uint32_t)fp, 7) : claim6(words + r * 8, fp)))
                 continue;
-            const unsigned long long j = atomicAdd(listN, 1ull);
+            const unsigned long long j = list_place(listN);
             if (j < listCap)
                 list[j] = code | (!places ? mz::kNoPlace : a ? mz::kSecondPlace : 0ull);
         }
@@ -261,12 +274,13 @@ __global__ void k_spill(uint64_t *__restrict__ list, const unsigned long long *_
 {
     const uint64_t n = *listN <= listCap ? *listN : 0;
     const bool b8 = g.format == FMT_B8X32 || g.format == FMT_MZ8, mz = is_mz(g.format);
+    uint32_t stashed = 0;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
          i += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t entry = list[i], code = mz ? entry & ~(mz::kSecondPlace | mz::kNoPlace) : entry;
         if (mz && (entry & mz::kNoPlace)) {
             list[i] = code;
-            atomicAdd(stashN, 1ull);
+            ++stashed;
             continue;
         }
         uint64_t rr[2], ff[2];
@@ -287,8 +301,7 @@ __global__ void k_spill(uint64_t *__restrict__ list, const unsigned long long *_
                 reach = d == 1 ? 1 : 2;
         }
         list[i] = reach == 3 ? code : STASH_EMPTY;
-        if (reach == 3)
-            atomicAdd(stashN, 1ull);
+        stashed += reach == 3;
         if (!mz)
             reach = 1; // hash buckets: the marker (B8_OVERFLOW, flag bit 0) means the stash
         if (b8)
@@ -296,6 +309,9 @@ __global__ void k_spill(uint64_t *__restrict__ list, const unsigned long long *_
         else
             atomicOr(home + 7, reach << 24); // 1 | 2 reads as 3: one place more is looked at
     }
+    stashed = __reduce_add_sync(0xffffffffu, stashed);
+    if ((threadIdx.x & 31) == 0 && stashed)
+        atomicAdd(stashN, (unsigned long long)stashed);
 }
 
 __global__ void k_stash(const uint64_t *__restrict__ list, uint64_t n, uint64_t *__restrict__ stash,
@@ -426,11 +442,15 @@ static ibs_status build_from_device_codes(ibs_table *t, const uint64_t *dCodes, 
     uint64_t *list = nullptr;
     uint32_t *left = nullptr;
     unsigned long long counts[2] = {0, 0};
-    // about 2% of the keys find no slot at the default loads; a table that
-    // leaves more (a forced load, many duplicates) is filled again with a list
-    // of the size that it then needs (which of several equal keys are listed
-    // can differ from pass to pass), at most of every place of every key
-    uint64_t listCap = n / 16 + 4096;
+    // The list has room for the keys that hash buckets leave (2.4% at the default
+    // load, 40% at 12 keys a bucket), and a little more; minimizer lines leave
+    // about 2% at theirs. A table that leaves more (a forced load of lines, many
+    // duplicates) is filled again with a list of the size that it then needs
+    // (which of several equal keys are listed can differ from pass to pass), at
+    // most of every place of every key. (Filled twice, 66M keys
+    // at 8 a bucket took 11.6 ms, filled once 7.7.)
+    const double share = is_mz(g.format) ? 1.0 / 16 : overflow_fraction((double)n / (double)nb, b8 ? 7 : 6) * 1.02 + 1.0 / 64;
+    uint64_t listCap = (uint64_t)((double)n * share) + 4096;
     const uint64_t most = n * (is_mz(g.format) ? 2 : 1) + 4096;
     for (int attempt = 0;; ++attempt) {
         void *mem = nullptr;
