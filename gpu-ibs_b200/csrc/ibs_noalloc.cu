@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(256) k_na_spans(TableView t, const uint64_t *_
 
 // Minimizer-line tables: the window scan's located blocks (mz_scan.cuh). A
 // lane that looks for its k-mer's minimizer alone hashes w m-mers a position:
-// 250 Mbp at k = 25 took 6.8 ms so, 1.7 ms this way.
+// 250 Mbp at k = 25 took 6.8 ms so, 1.8 ms this way.
 template <uint32_t K, uint32_t SEC>
 __global__ void __launch_bounds__(256, 3) k_na_spans_mz(const __grid_constant__ TableView t,
                                                         const uint64_t *__restrict__ seq,

@@ -1031,9 +1031,12 @@ extern "C" ibs_status ibs_scan_packed(ibs_table *t, const uint64_t *seq2bit,
     const bool pinnedIn = is_pinned(seq2bit) && is_pinned(nmask);
     // window groups: the first 1/128 of the reference (at least 4 Mbase), so
     // that the scan starts after a short copy, then each group 1.3x the one
-    // before (a copy of the next group takes no longer than the scan of the
-    // current one: host-to-device bandwidth carries about 1.35x the scan's
-    // bases per second) up to 1/8 of the reference
+    // before, up to 1/8 of the reference. Over hash buckets the upload (40 GB/s
+    // from pinned memory, 107 G bases/s) is 1.6x as fast as the scan, so a group
+    // arrives before the scan of the one before has ended; over minimizer lines
+    // (158 G positions/s) it is the slower of the two, and the groups bound the
+    // scan that is left after the last copy. (Groups that shrink again towards
+    // the end took 4.05 ms for 400 Mbp against 3.83: more and smaller copies.)
     const uint64_t totalBases = (seqWords - 1) * 32;
     const uint64_t maxGroup = std::max<uint64_t>(totalBases / 8 + 1, 16ull << 20);
     std::vector<uint64_t> gWin; // first window of each group
